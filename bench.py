@@ -42,7 +42,7 @@ WORKLOADS = {
     "c3": ("C[a,b,i,j]=sum_cd V[a,b,c,d]*T[c,d,i,j]; a..d extent 96 in blocks of 24-48, i,j 12 in 8-16 "
            "(the configuration's extents x 1/8); V block kept iff exp(-0.5 spread) >= 0.1; product screening 1e-10"),
 }
-FORM_KERNEL = {"plain": "k_contract_tiles", "batched": "k_matform + k_batched", "split": "k_slice + k_split"}
+FORM_KERNEL = {"plain": "k_tiles", "batched": "k_tiles", "split": "k_slice + k_split"}
 
 
 def parse():
@@ -517,13 +517,9 @@ def roofline_of(fname, flops, kern_ms, peaks, S=7):
                                      "frac": ach / peaks["split_pipe"] if peaks.get("split_pipe") else None,
                                      "peak_source": "the split kernel's stage copies (from L2) and 7-slice MMA "
                                                     "triangle alone, no epilogue (sht_measure_peak 3), this run"}}
-    if fname == "batched":
-        pk = peaks.get("dmma")
-        return {"bound": "tensor", "pipe": "fp64 tensor core (mma.sync m8n8k4)", "achieved": tf, "peak": pk,
-                "unit": "TFLOP/s", "frac": tf / pk if pk else None}
-    pk = peaks.get("fp64")
-    return {"bound": "tensor", "pipe": "fp64 FMA (DFMA)", "achieved": tf, "peak": pk, "unit": "TFLOP/s",
-            "frac": tf / pk if pk else None}
+    pk = peaks.get("dmma")
+    return {"bound": "tensor", "pipe": "fp64 tensor core (mma.sync m8n8k4)", "achieved": tf, "peak": pk,
+            "unit": "TFLOP/s", "frac": tf / pk if pk else None}
 
 
 def workload_leg(sht, ctx, w, forms, steps, warmup, stream, T, barrier, max_over_ranks, world, peaks,

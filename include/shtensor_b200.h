@@ -237,7 +237,7 @@ typedef struct {
   int64_t npairs;        /* block products after screening */
   double flops;          /* 2*m*n*k summed over the pairs */
   double queue_ms;       /* submit -> planning starts */
-  double plan_ms;        /* planning (matching, C pattern, work list, matrix-form layout) */
+  double plan_ms;        /* planning (matching, C pattern, work list; split form: slices) */
   double run_ms;         /* launch -> completion observed */
   double gpu_ms;         /* device time of its launch: the exec stream reaching it -> done */
   double latency_ms;     /* submit -> completion observed */

@@ -1,12 +1,11 @@
-// batched.cu -- the batched FP64 form: one persistent kernel over a size-class work list.
+// batched.cu -- the FP64 forms of the block-sparse contraction: one persistent kernel (tile_ring.cuh)
+// over a work list.
 //
-// Products run on the FP64 tensor cores (mma.sync m8n8k4, bit-identical to the fma chain).
-// Every C block is put in a size class by its matrix extents (m, n); each class has a tile
-// shape (picked by the autotuner, or by a padded-area model until tuned).  The plan builds a
-// single work list of (C block, tile, shape) items ordered by estimated cost, heaviest first;
-// a persistent grid of 128-thread CTAs (SMs x resident CTAs) pulls items from an atomic
-// counter and runs the pipelined tile (tile_pipe.cuh) of the item's shape.  Execute is a
-// counter reset plus one launch, and is what sht_plan_execute_graph captures.
+// Every C block gets a tile shape from its matrix extents (m, n): by a padded-area model, or, in
+// the batched form, by the autotuner's choice for its size class.  The plan builds a single work
+// list of (C block, tile, shape) items ordered by estimated cost, heaviest first; a persistent
+// grid (SMs x resident CTAs) claims items from an atomic counter.  Execute is a counter reset
+// plus one launch, and is what sht_plan_execute_graph captures.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -19,118 +18,42 @@
 
 #include "contract.h"
 #include "device_common.cuh"
-#include "tile_pipe.cuh"
+#include "tile_ring.cuh"
 
 namespace sht {
 
-// tile shapes (all 128 threads); few, so the persistent kernel's code stays in cache
-using B0 = PipeCfg<64, 64, 2>;   // 2x2 warps of 32x32
-using B1 = PipeCfg<128, 32, 4>;  // 4x1 warps of 32x32
-using B2 = PipeCfg<32, 128, 1>;  // 1x4 warps of 32x32
-using B3 = PipeCfg<128, 16, 4>;  // 4x1 warps of 32x16
-constexpr int kNumB = 4;
-static const int kBTM[kNumB] = {64, 128, 32, 128};
-static const int kBTN[kNumB] = {64, 32, 128, 16};
-
-constexpr size_t smax(size_t a, size_t b) { return a > b ? a : b; }
-constexpr size_t kBatchedSmem =
-    smax(smax(sizeof(PipeSmem<B0>), sizeof(PipeSmem<B1>)), smax(sizeof(PipeSmem<B2>), sizeof(PipeSmem<B3>)));
-
-struct BatchedArgs {
-  TileMaps mp;
-  TileScalars<double> sc;
-  const double* Am; const long long* aoff; const int* ald; const int* ak4;  // A in matrix form
-  const double* Bm; const long long* boff; const int* bld;                  // B in matrix form
-  double* C; const long long* offC; const int* dimsC;
-  const int* pair_a; const int* pair_b; const int* pstart;
-  const int4* work;
-  int nwork;
-  int* counter;
-  // serving launch: the requests' descriptors; request r owns launch items
-  // [multi[r].first, multi[r].first + multi[r].nwork)
-  const BatchedArgs* multi;
-  int nmulti;
-  int first;
-};
-
-template <class Cfg>
-__device__ __forceinline__ void run_item(const BatchedArgs& g, int4 w, unsigned char* smem) {
-  PipeSmem<Cfg>& sm = *reinterpret_cast<PipeSmem<Cfg>*>(smem);
-  const int c = w.x;
-  auto getc = [&](double*& p, const int*& d) {
-    p = g.C + g.offC[c];
-    d = g.dimsC + (long long)c * g.mp.oC;
-  };
-  auto getpair = [&](int p, PairView& v) {
-    const int ia = g.pair_a[p], ib = g.pair_b[p];
-    v.a = g.Am + g.aoff[ia];
-    v.lda = g.ald[ia];
-    v.K4 = g.ak4[ia];
-    v.b = g.Bm + g.boff[ib];
-    v.ldb = g.bld[ib];
-  };
-  tile_run_pipe<Cfg>(g.mp, g.sc, w.y, getc, getpair, g.pstart[c], g.pstart[c + 1], sm);
-}
-
-// Persistent kernel: each CTA takes items off the shared counter until the list is drained.
-// kMulti: the work of several executes in one launch (serving); a launch item is mapped to
-// its request by a binary search over the requests' first items.
-template <bool kMulti>
-__global__ void __launch_bounds__(128, 4) k_batched(BatchedArgs g) {
-  extern __shared__ __align__(16) unsigned char smem[];
-  __shared__ int s_item, s_req;
-  for (;;) {
-    if (threadIdx.x == 0) {
-      const int item = atomicAdd(g.counter, 1);
-      s_item = item;
-      if (kMulti && item < g.nwork) {
-        int lo = 0, hi = g.nmulti - 1;  // last request whose first item <= item
-        while (lo < hi) {
-          const int mid = (lo + hi + 1) >> 1;
-          if (g.multi[mid].first <= item) lo = mid; else hi = mid - 1;
-        }
-        s_req = lo;
-      }
-    }
-    __syncthreads();
-    const int item = s_item;
-    const int req = kMulti ? s_req : 0;
-    __syncthreads();
-    if (item >= g.nwork) break;
-    if constexpr (kMulti) {
-      const BatchedArgs& r = g.multi[req];
-      const int4 w = r.work[item - r.first];
-      switch (w.z) {
-        case 0: run_item<B0>(r, w, smem); break;
-        case 1: run_item<B1>(r, w, smem); break;
-        case 2: run_item<B2>(r, w, smem); break;
-        default: run_item<B3>(r, w, smem); break;
-      }
-    } else {
-      const int4 w = g.work[item];
-      switch (w.z) {
-        case 0: run_item<B0>(g, w, smem); break;
-        case 1: run_item<B1>(g, w, smem); break;
-        case 2: run_item<B2>(g, w, smem); break;
-        default: run_item<B3>(g, w, smem); break;
-      }
-    }
-  }
-}
-
-// resident CTAs for the persistent grid (the same for both instantiations: same smem, bounds)
-static int batched_grid(sht_ctx* ctx) {
+// resident CTAs of the persistent grid (the same for all instances: same shared memory, bounds)
+static int ring_grid(sht_ctx* ctx) {
   static std::once_flag once;
-  static int per_sm = 1;
   std::call_once(once, [] {
-    SHT_CUDA(cudaFuncSetAttribute(k_batched<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBatchedSmem));
-    SHT_CUDA(cudaFuncSetAttribute(k_batched<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBatchedSmem));
-    int a = 0, b = 0;
-    SHT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, k_batched<false>, 128, kBatchedSmem));
-    SHT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_batched<true>, 128, kBatchedSmem));
-    per_sm = std::max(1, std::min(a, b));
+    for (auto* k : {k_tiles<kRingPlan>, k_tiles<kRingMulti>, k_tiles<kRingStack>}) {
+      SHT_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(RingSmem)));
+      int n = 0;
+      SHT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, kRingThreads, sizeof(RingSmem)));
+      if (n < kRingCtas) fail(SHT_ERR_STATE, "FP64 tile kernel: fewer resident CTAs than its design");
+    }
   });
-  return ctx->num_sms * per_sm;
+  return ctx->num_sms * kRingCtas;
+}
+
+constexpr long long kRingWaitLimit = 1LL << 22;  // about a second
+
+// addressing flags of an expression (tile_ring.cuh)
+static bool consecutive(const int* x, int n) {
+  for (int t = 1; t < n; ++t)
+    if (x[t] != x[t - 1] + 1) return false;
+  return true;
+}
+static int ring_flags(const TileMaps& mp, const double* A, const double* B) {
+  const bool al = reinterpret_cast<uintptr_t>(A) % 16 == 0, bl = reinterpret_cast<uintptr_t>(B) % 16 == 0;
+  int f = 0;
+  if (al && consecutive(mp.row.x, mp.row.n) && consecutive(mp.kk.x, mp.kk.n))
+    f |= kRingLinA | (mp.kk.n && mp.kk.x[0] == 0 ? kRingKmA : 0);
+  if (bl && consecutive(mp.col.x, mp.col.n) && consecutive(mp.kk.y, mp.kk.n))
+    f |= kRingLinB | (mp.kk.n && mp.kk.y[0] == 0 ? kRingKmB : 0);
+  if (consecutive(mp.row.y, mp.row.n)) f |= kRingLinR;
+  if (consecutive(mp.col.y, mp.col.n)) f |= kRingLinC;
+  return f;
 }
 
 // ------------------------------------------------------------------ size classes
@@ -145,15 +68,22 @@ struct ClassKey {
   std::string str() const { return std::to_string(lm) + "," + std::to_string(ln) + "," + std::to_string(lk); }
 };
 
-// padded-area cost model: MACs the tile shape runs (padding included) + a per-tile cost
-static int model_shape(long long m, long long n) {
-  double best = 1e300;
+// Cost of one C block per unit of contracted extent in a tile shape, in products: what the tensor
+// pipe runs (the tile's fragments of 8x8, and four times the busiest warp's, averaged: a tile
+// waits for its busiest warp, but another CTA fills the gap), the operand copies, and a fixed
+// cost per tile.
+__host__ __device__ static inline float shape_cost(int m, int n, int sh) {
+  const int ntr = ring_ntiles(m, ring_tm(sh)), ntc = ring_ntiles(n, ring_tn(sh));
+  const int fr = ring_step(m, ntr) / 8, fc = ring_step(n, ntc) / 8;
+  const float busiest = 4.0f * (float)(((fr + 1) / 2) * ((fc + 1) / 2));
+  return (float)ntr * (float)ntc * (32.0f * ((float)(fr * fc) + busiest) + 64.0f * (float)(fr + fc) + 512.0f);
+}
+__host__ __device__ static inline int model_shape(int m, int n) {
+  float best = 3.0e38f;
   int bi = 0;
-  for (int s = 0; s < kNumB; ++s) {
-    const long long tm = kBTM[s], tn = kBTN[s];
-    const long long tiles = ((m + tm - 1) / tm) * ((n + tn - 1) / tn);
-    const double cost = (double)tiles * (double)(tm * tn) + 3072.0 * (double)tiles;
-    if (cost < best) { best = cost; bi = s; }
+  for (int s = 0; s < kRingShapes; ++s) {
+    const float c = shape_cost(m, n, s);
+    if (c < best) { best = c; bi = s; }
   }
   return bi;
 }
@@ -214,8 +144,8 @@ static void build_batched_work(sht_plan* p, const HostPlanView& v, const std::ma
   for (long long c = 0; c < nc; ++c) {
     if (subset && !(*subset)[c]) continue;
     auto it = shape_of.find(v.key[c].str());
-    const int sh = it != shape_of.end() ? it->second : model_shape(v.m[c], v.n[c]);
-    const long long tm = kBTM[sh], tn = kBTN[sh];
+    const int sh = it != shape_of.end() ? it->second : model_shape((int)v.m[c], (int)v.n[c]);
+    const long long tm = ring_tm(sh), tn = ring_tn(sh);
     const int tiles = (int)(((v.m[c] + tm - 1) / tm) * ((v.n[c] + tn - 1) / tn));
     const bool has = v.pstart[c + 1] > v.pstart[c];
     blks.push_back({has ? (double)tm * tn * (double)v.ksum[c] : -1.0, (int)c, sh, tiles, has});
@@ -226,7 +156,8 @@ static void build_batched_work(sht_plan* p, const HostPlanView& v, const std::ma
   std::vector<int4> w;
   w.reserve(nall);
   for (const Blk& b : blks)
-    for (int t = 0; t < b.tiles; ++t) w.push_back(make_int4(b.c, t, b.sh, 0));
+    for (int t = 0; t < b.tiles; ++t)
+      w.push_back(ring_item(b.c, t, (int)v.m[b.c], (int)v.n[b.c], ring_tm(b.sh), ring_tn(b.sh)));
   if (w.size() > (size_t)INT32_MAX) fail(SHT_ERR_UNSUPPORTED, "work list above 2^31 tiles");
   if (out) {
     *out = std::move(w);
@@ -241,20 +172,15 @@ static void build_batched_work(sht_plan* p, const HostPlanView& v, const std::ma
   }
 }
 
-static void launch_batched(sht_plan* p, BatchedArgs& b, cudaStream_t s) {
-  if (b.nwork <= 0) return;
-  SHT_CUDA(cudaMemsetAsync(b.counter, 0, sizeof(int), s));
-  const int grid = std::min<long long>(batched_grid(p->ctx), b.nwork);
-  k_batched<false><<<grid, 128, kBatchedSmem, s>>>(b);
+static void launch_plan(sht_ctx* ctx, const RingArgs& g, cudaStream_t s) {
+  if (g.nwork <= 0) return;
+  SHT_CUDA(cudaMemsetAsync(g.counter, 0, sizeof(int), s));
+  const int grid = std::min(ring_grid(ctx), g.nwork);
+  k_tiles<kRingPlan><<<grid, kRingThreads, sizeof(RingSmem), s>>>(g);
   SHT_CUDA(cudaGetLastError());
 }
 
 // ------------------------------------------------------------------ device work list
-struct ShapeSet {
-  int n;
-  int tm[kNumB], tn[kNumB];
-};
-
 __device__ __forceinline__ int ilog2ceil_dev(long long v) {
   int b = 0;
   while ((1LL << b) < v) ++b;
@@ -263,7 +189,7 @@ __device__ __forceinline__ int ilog2ceil_dev(long long v) {
 
 __global__ void k_block_shapes(const int* __restrict__ cm, const int* __restrict__ cn,
                                const long long* __restrict__ cksum, const int* __restrict__ pstart, long long nc,
-                               const unsigned char* __restrict__ table, int fixed_tm, int fixed_tn, ShapeSet ss,
+                               const unsigned char* __restrict__ table, int fixed_tm, int fixed_tn,
                                int* __restrict__ shape, long long* __restrict__ tiles,
                                long long* __restrict__ touched_tiles, unsigned long long* __restrict__ key,
                                int* __restrict__ idx) {
@@ -271,7 +197,6 @@ __global__ void k_block_shapes(const int* __restrict__ cm, const int* __restrict
     const long long m = cm[c], n = cn[c], ks = cksum[c];
     const int np = pstart[c + 1] - pstart[c];
     int sh = 0;
-    long long tm = fixed_tm, tn = fixed_tn;
     if (fixed_tm <= 0) {
       int t = 255;
       if (table) {
@@ -279,20 +204,9 @@ __global__ void k_block_shapes(const int* __restrict__ cm, const int* __restrict
         const int lk = min(ilog2ceil_dev(np > 0 ? (ks / np > 0 ? ks / np : 1) : 1), 31);
         t = table[(lm * 32 + ln) * 32 + lk];
       }
-      if (t != 255) {
-        sh = t;
-      } else {  // padded-area model, as on the host
-        double best = 1e300;
-        for (int q = 0; q < ss.n; ++q) {
-          const long long a = ss.tm[q], b = ss.tn[q];
-          const long long nt = ((m + a - 1) / a) * ((n + b - 1) / b);
-          const double cost = (double)nt * (double)(a * b) + 3072.0 * (double)nt;
-          if (cost < best) { best = cost; sh = q; }
-        }
-      }
-      tm = ss.tm[sh];
-      tn = ss.tn[sh];
+      sh = t != 255 ? t : model_shape((int)m, (int)n);
     }
+    const long long tm = fixed_tm > 0 ? fixed_tm : ring_tm(sh), tn = fixed_tm > 0 ? fixed_tn : ring_tn(sh);
     const long long nt = ((m + tm - 1) / tm) * ((n + tn - 1) / tn);
     shape[c] = sh;
     tiles[c] = nt;
@@ -311,13 +225,17 @@ __global__ void k_gather_tiles(const int* __restrict__ idx, const long long* __r
     out[i] = tiles[idx[i]];
 }
 
+// One warp per C block of the order: its tiles, as (C block, tile, ., .) for split plans (ring 0).
 __global__ void k_emit_items(const int* __restrict__ idx, const long long* __restrict__ tiles_sorted,
-                             const long long* __restrict__ off, const int* __restrict__ shape, long long nc,
+                             const long long* __restrict__ off, const int* __restrict__ shape,
+                             const int* __restrict__ cm, const int* __restrict__ cn, int ring, long long nc,
                              int4* __restrict__ work) {
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < nc; i += (long long)gridDim.x * blockDim.x) {
-    const int c = idx[i];
-    const long long w0 = off[i];
-    for (long long t = 0; t < tiles_sorted[i]; ++t) work[w0 + t] = make_int4(c, (int)t, shape[c], 0);
+  const int lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
+  for (long long i = (long long)blockIdx.x * wpb + (threadIdx.x >> 5); i < nc; i += (long long)gridDim.x * wpb) {
+    const int c = idx[i], sh = shape[c], m = cm[c], n = cn[c];
+    const long long w0 = off[i], nt = tiles_sorted[i];
+    for (long long t = lane; t < nt; t += 32)
+      work[w0 + t] = ring ? ring_item(c, (int)t, m, n, ring_tm(sh), ring_tn(sh)) : make_int4(c, (int)t, 0, 0);
   }
 }
 
@@ -342,9 +260,6 @@ void device_work_list(sht_plan* p, int fixed_tm, int fixed_tn, bool per_class, c
     p->d_bwork = PoolBuf(pool, sizeof(int4), s);
     return;
   }
-  ShapeSet ss{};
-  ss.n = kNumB;
-  for (int q = 0; q < kNumB; ++q) { ss.tm[q] = kBTM[q]; ss.tn[q] = kBTN[q]; }
   PoolBuf table;
   if (per_class && !p->ctx->tuned.empty()) {
     std::vector<unsigned char> h(32 * 32 * 32, 255);
@@ -362,7 +277,7 @@ void device_work_list(sht_plan* p, int fixed_tm, int fixed_tn, bool per_class, c
       off(pool, nc * 8, s), sums(pool, 16, s);
   k_block_shapes<<<grid_for(nc, 256), 256, 0, s>>>(
       p->d_cm.as<int>(), p->d_cn.as<int>(), p->d_cksum.as<long long>(), p->d_pstart.as<int>(), nc,
-      table.as<unsigned char>(), per_class ? 0 : fixed_tm, fixed_tn, ss, shape.as<int>(), tiles.as<long long>(),
+      table.as<unsigned char>(), fixed_tm, fixed_tn, shape.as<int>(), tiles.as<long long>(),
       ttiles.as<long long>(), key.as<unsigned long long>(), idx.as<int>());
   SHT_CUDA(cudaGetLastError());
   // a caller's order (ascending keys, untouched blocks keyed last) replaces the cost order
@@ -424,51 +339,47 @@ void device_work_list(sht_plan* p, int fixed_tm, int fixed_tn, bool per_class, c
   p->bwork = total;
   p->bwork_touched = h[1];
   p->d_bwork = PoolBuf(pool, std::max(total, 1LL) * sizeof(int4), s);
-  k_emit_items<<<grid_for(nc, 128), 128, 0, s>>>(idx2.as<int>(), tsorted.as<long long>(), off.as<long long>(),
-                                                  shape.as<int>(), nc, p->d_bwork.as<int4>());
+  k_emit_items<<<grid_for(nc * 32, 128), 128, 0, s>>>(idx2.as<int>(), tsorted.as<long long>(), off.as<long long>(),
+                                                      shape.as<int>(), p->d_cm.as<int>(), p->d_cn.as<int>(),
+                                                      fixed_tm > 0 ? 0 : 1, nc, p->d_bwork.as<int4>());
   SHT_CUDA(cudaGetLastError());
 }
 
-void batched_prepare(sht_plan* p, cudaStream_t s) {
+void ring_prepare(sht_plan* p, cudaStream_t s) {
   p->d_counter = PoolBuf(p->ctx->pool.get(), 256, s);
-  matform_prepare(p, s);
-  trace("batched: matform layout", s);
-  device_work_list(p, 0, 0, true, s);
-  trace("batched: work list", s);
+  device_work_list(p, 0, 0, p->mode == SHT_MODE_BATCHED_FP64, s);
+  trace("work list", s);
 }
 
-
-static void fill_operands(sht_plan* p, BatchedArgs& b) {
-  b.Am = p->mf_a.as<double>(); b.aoff = p->mf_aoff.as<long long>(); b.ald = p->mf_ald.as<int>();
-  b.ak4 = p->mf_ak4.as<int>();
-  b.Bm = p->mf_b.as<double>(); b.boff = p->mf_boff.as<long long>(); b.bld = p->mf_bld.as<int>();
-}
-
-// Descriptor of one batched plan's execute (also used by the serving loop).
-static BatchedArgs batched_args(sht_plan* p, const SparseArgs& g) {
-  BatchedArgs b{};
-  b.mp = g.mp;
-  b.sc = g.sc;
-  fill_operands(p, b);
-  b.C = g.C; b.offC = g.offC; b.dimsC = g.dimsC;
-  b.pair_a = g.pair_a; b.pair_b = g.pair_b; b.pstart = g.pstart;
-  b.work = p->d_bwork.as<int4>();
+// The kernel arguments of one plan's execute (also used by the serving loop).
+static RingArgs ring_args(sht_plan* p, const SparseArgs& g) {
+  RingArgs r{};
+  r.mp = g.mp;
+  r.sc = g.sc;
+  r.flags = ring_flags(g.mp, g.A, g.B);
+  r.A = g.A; r.offA = g.offA; r.dimsA = g.dimsA;
+  r.B = g.B; r.offB = g.offB; r.dimsB = g.dimsB;
+  r.C = g.C; r.offC = g.offC; r.dimsC = g.dimsC;
+  r.recs = g.recs; r.pstart = g.pstart;
+  r.work = p->d_bwork.as<int4>();
   uint64_t one, bb;
   const double d1 = 1.0;
   std::memcpy(&one, &d1, 8);
   std::memcpy(&bb, &g.sc.beta, 8);
-  b.nwork = (int)((bb == one) ? p->bwork_touched : p->bwork);
-  b.counter = p->d_counter.as<int>();
-  return b;
+  r.nwork = (int)((bb == one) ? p->bwork_touched : p->bwork);
+  r.counter = p->d_counter.as<unsigned>();
+  r.err = ctx_error_word(p->ctx);
+  r.wait_limit = kRingWaitLimit;
+  return r;
 }
 
-size_t batched_desc_bytes() { return sizeof(BatchedArgs); }
+size_t batched_desc_bytes() { return sizeof(RingArgs); }
 
 // resident CTAs per SM of the persistent kernel
-int batched_ctas_per_sm(sht_ctx* ctx) { return batched_grid(ctx) / ctx->num_sms; }
+int batched_ctas_per_sm(sht_ctx* ctx) { return ring_grid(ctx) / ctx->num_sms; }
 
-// One persistent launch over the work of several batched executes (the serving loop).  The
-// operands must already be in matrix form (matform_execute).  host_descs: pinned host memory
+// One persistent launch over the work of several batched executes (the serving loop).
+// host_descs: pinned host memory
 // for plans.size() descriptors that the caller keeps unchanged until the launch completes (the
 // upload reads it asynchronously); `descs` and `counter` are allocated on `s` and must be held
 // as long.  ctas_per_sm (1..batched_ctas_per_sm) sets the persistent grid: fewer than the
@@ -477,42 +388,34 @@ int batched_ctas_per_sm(sht_ctx* ctx) { return batched_grid(ctx) / ctx->num_sms;
 long long batched_multi_launch(sht_ctx* ctx, const std::vector<sht_plan*>& plans, const std::vector<SparseArgs>& args,
                                void* host_descs, PoolBuf& descs, PoolBuf& counter, int ctas_per_sm, cudaStream_t s) {
   DevicePool* pool = ctx->pool.get();
-  BatchedArgs* h = static_cast<BatchedArgs*>(host_descs);
+  RingArgs* h = static_cast<RingArgs*>(host_descs);
   long long total = 0;
   for (size_t i = 0; i < plans.size(); ++i) {
-    h[i] = batched_args(plans[i], args[i]);
+    h[i] = ring_args(plans[i], args[i]);
     h[i].first = (int)total;
     total += h[i].nwork;
     if (total > (long long)INT32_MAX) fail(SHT_ERR_UNSUPPORTED, "batched launch above 2^31 tiles");
   }
   if (total == 0) return 0;
-  descs = PoolBuf(pool, plans.size() * sizeof(BatchedArgs), s);
+  descs = PoolBuf(pool, plans.size() * sizeof(RingArgs), s);
   counter = PoolBuf(pool, 256, s);
-  SHT_CUDA(cudaMemcpyAsync(descs.ptr, h, plans.size() * sizeof(BatchedArgs), cudaMemcpyHostToDevice, s));
-  BatchedArgs b = h[0];
+  SHT_CUDA(cudaMemcpyAsync(descs.ptr, h, plans.size() * sizeof(RingArgs), cudaMemcpyHostToDevice, s));
+  RingArgs b = h[0];
   b.nwork = (int)total;
-  b.counter = counter.as<int>();
-  b.multi = descs.as<BatchedArgs>();
+  b.counter = counter.as<unsigned>();
+  b.multi = descs.as<RingArgs>();
   b.nmulti = (int)plans.size();
   SHT_CUDA(cudaMemsetAsync(b.counter, 0, sizeof(int), s));
   const int per_sm = std::max(1, std::min(ctas_per_sm, batched_ctas_per_sm(ctx)));
   const int grid = (int)std::min<long long>((long long)ctx->num_sms * per_sm, total);
-  k_batched<true><<<grid, 128, kBatchedSmem, s>>>(b);
+  k_tiles<kRingMulti><<<grid, kRingThreads, sizeof(RingSmem), s>>>(b);
   SHT_CUDA(cudaGetLastError());
   return total;
 }
 
-void batched_launch(sht_plan* p, const SparseArgs& g, cudaStream_t s) {
-  BatchedArgs b = batched_args(p, g);
-  launch_batched(p, b, s);
-}
-
-void batched_execute(sht_plan* p, const SparseArgs& g, long long, cudaStream_t s) {
-  BatchedArgs b = batched_args(p, g);
-  if (!g.sc.alpha_zero) matform_execute(p, g.sc.alpha, s);
-  trace("batched: matform kernels", s);
-  launch_batched(p, b, s);
-  trace("batched: tile kernel", s);
+void ring_launch(sht_plan* p, const SparseArgs& g, cudaStream_t s) {
+  launch_plan(p->ctx, ring_args(p, g), s);
+  trace("tile kernel", s);
 }
 
 // ------------------------------------------------------------------ autotuner
@@ -530,10 +433,9 @@ void autotune(sht_plan* p, const char* cache_file, cudaStream_t s) {
     std::string g, k;
     int sh;
     while (in >> g >> k >> sh)
-      if (g == gpu && sh >= 0 && sh < kNumB) ctx->tuned[k] = sh;
+      if (g == gpu && sh >= 0 && sh < kRingShapes) ctx->tuned[k] = sh;
   }
   const HostPlanView v = host_view(p, s);
-  matform_execute(p, 1.0, s);  // operands in matrix form for the timing runs
   std::map<std::string, std::vector<long long>> members;
   for (long long c = 0; c < p->ncblk; ++c)
     if (v.pstart[c + 1] > v.pstart[c]) members[v.key[c].str()].push_back(c);
@@ -559,27 +461,24 @@ void autotune(sht_plan* p, const char* cache_file, cudaStream_t s) {
     PoolBuf scratch(pool, std::max(elems, 1LL) * 8, s), doffs(pool, p->ncblk * 8, s), work(pool, 1, s);
     SHT_CUDA(cudaMemcpyAsync(doffs.ptr, offs.data(), p->ncblk * 8, cudaMemcpyHostToDevice, s));
     double best = 1e300;
-    int best_sh = model_shape(v.m[kv.second[0]], v.n[kv.second[0]]);
-    for (int sh = 0; sh < kNumB; ++sh) {
+    int best_sh = model_shape((int)v.m[kv.second[0]], (int)v.n[kv.second[0]]);
+    for (int sh = 0; sh < kRingShapes; ++sh) {
       std::map<std::string, int> forced{{kv.first, sh}};
       std::vector<int4> items;
       build_batched_work(p, v, forced, s, &subset, &items);
       work = PoolBuf(pool, items.size() * sizeof(int4), s);
       SHT_CUDA(cudaMemcpyAsync(work.ptr, items.data(), items.size() * sizeof(int4), cudaMemcpyHostToDevice, s));
-      BatchedArgs b{};
-      b.mp = p->tmaps;
-      b.sc = {1.0, 0.0, 1, 0};
-      fill_operands(p, b);
-      b.C = scratch.as<double>(); b.offC = doffs.as<long long>(); b.dimsC = p->C->d_dims.as<int>();
-      b.pair_a = p->d_pair_a.as<int>(); b.pair_b = p->d_pair_b.as<int>(); b.pstart = p->d_pstart.as<int>();
+      SparseArgs sa = sparse_args(p, 1.0, 0.0);
+      sa.C = scratch.as<double>();
+      sa.offC = doffs.as<long long>();
+      RingArgs b = ring_args(p, sa);
       b.work = work.as<int4>();
       b.nwork = (int)items.size();
-      b.counter = p->d_counter.as<int>();
-      launch_batched(p, b, s);  // warm-up
+      launch_plan(ctx, b, s);  // warm-up
       float ms = 0, tot = 0;
       for (int r = 0; r < 3; ++r) {
         SHT_CUDA(cudaEventRecord(e0, s));
-        launch_batched(p, b, s);
+        launch_plan(ctx, b, s);
         SHT_CUDA(cudaEventRecord(e1, s));
         SHT_CUDA(cudaEventSynchronize(e1));
         SHT_CUDA(cudaEventElapsedTime(&ms, e0, e1));

@@ -78,47 +78,43 @@ static void contract_split(sht_plan* p, double alpha, double beta, cudaStream_t 
   trace("contract: split kernel launched", s);
 }
 
-// A bounded wait of an earlier split launch on this context ran out: report it at this call.
+// A bounded wait of an earlier launch on this context ran out: report it at this call.
 static void raise_pending(sht_ctx* ctx) {
   if (const int e = ctx_take_error(ctx))
-    fail((sht_status)e, "an earlier split-precision launch on this context failed: a bounded wait on the tensor "
-                        "cores expired (its result is undefined)");
+    fail((sht_status)e, "an earlier launch on this context failed: a bounded wait of its kernel expired (its result "
+                        "is undefined)");
 }
 
-// Batched form of sht_contract, overlapped the same way: the matrix form of A and B (patterns
-// and values of A and B only) on the caller's stream, the plan and its size-class work list on
-// the lane stream.
-static void contract_batched(sht_plan* p, double alpha, double beta, cudaStream_t s) {
+// Plan-time work of a form after plan_build.
+static void prepare_mode(sht_plan* p, cudaStream_t s) {
+  if (p->mode == SHT_MODE_SPLIT) split_prepare(p, p->ctx->split_slices ? p->ctx->split_slices : split_slices_default(), s);
+  else ring_prepare(p, s);
+}
+
+// The FP64 forms of sht_contract.  The build reads indices only (complete: every index change in
+// this library returns after it is done) unless it screens, so it runs on a lane stream and a
+// contraction into a C whose pattern holds the product plans while earlier work on s still runs.
+static void contract_fp64(sht_plan* p, double alpha, double beta, cudaStream_t s) {
   sht_ctx* ctx = p->ctx;
   LaneLease lane(ctx);
   const cudaStream_t ps = lane.lane.stream;
   SHT_CUDA(cudaEventRecord(lane.lane.start, s));
-  p->d_counter = PoolBuf(ctx->pool.get(), 256, s);
-  matform_prepare(p, s);
-  uint64_t ab;
-  std::memcpy(&ab, &alpha, 8);
-  if (ab != 0) matform_execute(p, alpha, s);
-  trace("contract: matrix form launched", s);
-  // as in the split form: the build waits for earlier work on s only when it reads values
   if (p->eps > 0.0) SHT_CUDA(cudaStreamWaitEvent(ps, lane.lane.start, 0));
   try {
     plan_build(p, ps, true);
-    device_work_list(p, 0, 0, true, ps);
+    ring_prepare(p, ps);
   } catch (const PatternGrew&) {
+    // the product adds blocks to C: build again, growing C's pattern, which moves C's values
+    // (after earlier work on s has written them)
     SHT_CUDA(cudaStreamWaitEvent(ps, lane.lane.start, 0));
     plan_build(p, ps, false);
-    device_work_list(p, 0, 0, true, ps);
+    ring_prepare(p, ps);
   }
   SHT_CUDA(cudaEventRecord(lane.lane.done, ps));
   SHT_CUDA(cudaStreamWaitEvent(s, lane.lane.done, 0));
   plan_touch(p, s);
-  batched_launch(p, sparse_args(p, alpha, beta), s);
-  trace("contract: batched kernel launched", s);
-}
-
-static void prepare_mode(sht_plan* p, cudaStream_t s) {
-  if (p->mode == SHT_MODE_BATCHED_FP64) batched_prepare(p, s);
-  if (p->mode == SHT_MODE_SPLIT) split_prepare(p, p->ctx->split_slices ? p->ctx->split_slices : split_slices_default(), s);
+  ring_launch(p, sparse_args(p, alpha, beta), s);
+  trace("contract: tile kernel launched", s);
 }
 
 volatile int* ctx_error_word(sht_ctx* ctx) {
@@ -490,7 +486,7 @@ sht_status sht_plan_create(sht_ctx* ctx, const char* expr, sht_tensor* A, sht_te
 sht_status sht_plan_execute(sht_plan* p, double alpha, double beta, void* stream) {
   return guard([&] {
     need(p, "null plan");
-    if (p->mode == SHT_MODE_SPLIT) raise_pending(p->ctx);
+    raise_pending(p->ctx);
     plan_execute(p, alpha, beta, as_stream(stream));
   });
 }
@@ -532,7 +528,7 @@ sht_status sht_plan_report(sht_plan* p, sht_contract_report* rep) {
     rep->npairs = p->npairs;
     rep->nblocks_c = p->C->nblocks;
     rep->nnz_c = p->C->nnz;
-    rep->nwork = p->mode == SHT_MODE_BATCHED_FP64 ? p->bwork : p->nwork;
+    rep->nwork = p->mode == SHT_MODE_SPLIT ? 0 : p->bwork;
     rep->flops = plan_flops(p, p->ctx->stage_stream);  // waits for the count's own event
     rep->plan_ms = p->plan_ms;
     rep->exec_ms = p->exec_ms;
@@ -575,24 +571,16 @@ sht_status sht_contract(sht_ctx* ctx, const char* expr, double alpha, sht_tensor
     need(norm >= SHT_NORM_FROBENIUS && norm <= SHT_NORM_FROBENIUS_REFCOMPAT, "unknown norm");
     cudaStream_t s = as_stream(stream);
     std::unique_ptr<sht_plan> p;
-    if (mode == SHT_MODE_SPLIT) raise_pending(ctx);
-    if (mode == SHT_MODE_SPLIT) {
-      p.reset(plan_init(ctx, expr, A, B, C, eps, norm, mode, s));
-      contract_split(p.get(), alpha, beta, s);
-    } else if (mode == SHT_MODE_BATCHED_FP64) {
-      p.reset(plan_init(ctx, expr, A, B, C, eps, norm, mode, s));
-      contract_batched(p.get(), alpha, beta, s);
-    } else {
-      p.reset(plan_create(ctx, expr, A, B, C, eps, norm, mode, s));
-      prepare_mode(p.get(), s);
-      plan_execute(p.get(), alpha, beta, s);
-    }
+    raise_pending(ctx);
+    p.reset(plan_init(ctx, expr, A, B, C, eps, norm, mode, s));
+    if (mode == SHT_MODE_SPLIT) contract_split(p.get(), alpha, beta, s);
+    else contract_fp64(p.get(), alpha, beta, s);
     if (rep) {
       std::memset(rep, 0, sizeof(*rep));
       rep->npairs = p->npairs;
       rep->nblocks_c = C->nblocks;
       rep->nnz_c = C->nnz;
-      rep->nwork = p->mode == SHT_MODE_BATCHED_FP64 ? p->bwork : p->nwork;
+      rep->nwork = p->mode == SHT_MODE_SPLIT ? 0 : p->bwork;
       rep->flops = plan_flops(p.get(), s);
       rep->plan_ms = p->plan_ms;
       rep->slices = p->split_slices;

@@ -1,4 +1,4 @@
-// contract.cu -- block-sparse contraction on one GPU: device plan + FP64 tile kernels.
+// contract.cu -- block-sparse contraction on one GPU: the device plan.
 //
 // Plan (all on the device; the reference has no block-sparse contract, src/Tensor/Tensor.cpp
 // is empty, so the rules below are this library's canonical ones, restated in the oracle):
@@ -10,9 +10,9 @@
 //   3. a stable radix sort by idC gives the canonical pair order (idC, idA, idB);
 //   4. the distinct idC merged with C's stored ids is the result pattern; C is re-reserved
 //      to it when it grows (old blocks copied, new blocks zero-filled);
-//   5. per C block its pair range, and the work list of TM x TN tiles (tiles of C blocks
-//      with pairs first, untouched C blocks after; the latter are skipped when beta == 1).
-// Execute launches the output-stationary tile kernel (tile_core.cuh) over the work list.
+//   5. per C block its pair range; the form's work list of tiles follows (batched.cu, split.cu:
+//      tiles of C blocks with pairs first, untouched C blocks after; the latter are skipped
+//      when beta == 1).
 #include <cub/cub.cuh>
 
 #include <algorithm>
@@ -135,13 +135,52 @@ __global__ void k_emit(const unsigned long long* __restrict__ keyA, const long l
   }
 }
 
+// The operand side of the linear addressing of a block of extents d (tile_ring.cuh): strides of its
+// first free and first contracted mode, and the contracted extent.
+struct RecModes {
+  int order, fx, kx;
+  unsigned kmask;
+};
+__device__ __forceinline__ void rec_strides(const int* __restrict__ d, const RecModes& m, int& rs, int& ks, int& K) {
+  rs = ks = K = 1;
+#pragma unroll
+  for (int u = 0; u < kMaxOrder; ++u) {
+    const int e = u < m.order ? d[u] : 1;
+    if (u < m.fx) rs *= e;
+    if (u < m.kx) ks *= e;
+    if (m.kmask >> u & 1) K *= e;
+  }
+}
+
+// The pairs in canonical order, with their records when rec is given.
 __global__ void k_gather_pairs(const int* __restrict__ order, const int* __restrict__ pa_in, const int* __restrict__ pb_in,
-                               long long n, int* __restrict__ pa, int* __restrict__ pb) {
+                               long long n, int* __restrict__ pa, int* __restrict__ pb, PairRec* __restrict__ rec,
+                               RecModes ma, RecModes mb, const long long* __restrict__ offA,
+                               const int* __restrict__ dimsA, const long long* __restrict__ offB,
+                               const int* __restrict__ dimsB) {
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
     const int o = order[i];
-    pa[i] = pa_in[o];
-    pb[i] = pb_in[o];
+    const int ia = pa_in[o], ib = pb_in[o];
+    pa[i] = ia;
+    pb[i] = ib;
+    if (!rec) continue;
+    PairRec r;
+    int kb;
+    r.offA = offA[ia];
+    r.offB = offB[ib];
+    rec_strides(dimsA + (long long)ia * ma.order, ma, r.rsA, r.ksA, r.K);
+    rec_strides(dimsB + (long long)ib * mb.order, mb, r.rsB, r.ksB, kb);
+    r.ia = ia;
+    r.ib = ib;
+    r.pad = 0;
+    rec[i] = r;
   }
+}
+
+static RecModes rec_modes(int order, const std::vector<int>& free_modes, const std::vector<int>& k_modes) {
+  RecModes m{order, free_modes.empty() ? 0 : free_modes[0], k_modes.empty() ? 0 : k_modes[0], 0u};
+  for (int x : k_modes) m.kmask |= 1u << x;
+  return m;
 }
 
 // pair range of each C block
@@ -167,78 +206,7 @@ __global__ void k_move_blocks(const T* __restrict__ src, const long long* __rest
   }
 }
 
-// tiles per C block for a given tile shape; touched / untouched counted separately
-__global__ void k_tile_counts(const int* __restrict__ dimsC, int oC, ModeMap row, ModeMap col, long long nc,
-                              const int* __restrict__ pstart, int TM, int TN, long long* __restrict__ nt_touched,
-                              long long* __restrict__ nt_untouched) {
-  for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < nc; c += (long long)gridDim.x * blockDim.x) {
-    long long m = 1, n = 1;
-    for (int t = 0; t < row.n; ++t) m *= dimsC[c * oC + row.y[t]];
-    for (int t = 0; t < col.n; ++t) n *= dimsC[c * oC + col.y[t]];
-    const long long tiles = ((m + TM - 1) / TM) * ((n + TN - 1) / TN);
-    const bool touched = pstart[c + 1] > pstart[c];
-    nt_touched[c] = touched ? tiles : 0;
-    nt_untouched[c] = touched ? 0 : tiles;
-  }
-}
-
-__global__ void k_tile_emit(long long nc, const long long* __restrict__ cnt_t, const long long* __restrict__ off_t,
-                            const long long* __restrict__ cnt_u, const long long* __restrict__ off_u,
-                            long long base_u, int2* __restrict__ work) {
-  for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < nc; c += (long long)gridDim.x * blockDim.x) {
-    const long long nt = cnt_t[c] + cnt_u[c];
-    const long long w0 = cnt_t[c] ? off_t[c] : base_u + off_u[c];
-    for (long long t = 0; t < nt; ++t) work[w0 + t] = make_int2((int)c, (int)t);
-  }
-}
-
-// ---------------------------------------------------------------------------------------
-// execute kernels
-// ---------------------------------------------------------------------------------------
-template <class Cfg>
-__global__ void __launch_bounds__(Cfg::kThreads) k_contract_tiles(SparseArgs g) {
-  __shared__ TileSmem<double, Cfg> sm;
-  const int2 w = g.work[blockIdx.x];
-  const int c = w.x;
-  auto getc = [&](double*& p, const int*& d) {
-    p = g.C + g.offC[c];
-    d = g.dimsC + (long long)c * g.mp.oC;
-  };
-  auto getpair = [&](int p, const double*& a, const int*& ad, const double*& b, const int*& bd) {
-    const int ia = g.pair_a[p], ib = g.pair_b[p];
-    a = g.A + g.offA[ia];
-    ad = g.dimsA + (long long)ia * g.mp.oA;
-    b = g.B + g.offB[ib];
-    bd = g.dimsB + (long long)ib * g.mp.oB;
-  };
-  tile_run<double, Cfg>(g.mp, g.sc, w.y, getc, getpair, g.pstart[c], g.pstart[c + 1], sm);
-}
-
-// tile shapes of the plain path (256 or 128 threads)
-using Cfg64x64 = TileCfg<64, 64, 16, 4, 4>;
 using Cfg128x32 = TileCfg<128, 32, 16, 8, 2>;
-using Cfg32x128 = TileCfg<32, 128, 16, 2, 8>;
-using Cfg128x16 = TileCfg<128, 16, 16, 4, 4>;
-using Cfg16x128 = TileCfg<16, 128, 16, 4, 4>;
-using Cfg32x32 = TileCfg<32, 32, 16, 2, 2>;
-
-struct TileShape { int tm, tn; };
-static const TileShape kShapes[] = {{64, 64}, {128, 32}, {32, 128}, {128, 16}, {16, 128}, {32, 32}};
-constexpr int kNumShapes = 6;
-
-static void launch_tiles(int cfg, long long nwork, const SparseArgs& g, cudaStream_t s) {
-  if (nwork <= 0) return;
-  const unsigned grid = (unsigned)nwork;
-  switch (cfg) {
-    case 0: k_contract_tiles<Cfg64x64><<<grid, Cfg64x64::kThreads, 0, s>>>(g); break;
-    case 1: k_contract_tiles<Cfg128x32><<<grid, Cfg128x32::kThreads, 0, s>>>(g); break;
-    case 2: k_contract_tiles<Cfg32x128><<<grid, Cfg32x128::kThreads, 0, s>>>(g); break;
-    case 3: k_contract_tiles<Cfg128x16><<<grid, Cfg128x16::kThreads, 0, s>>>(g); break;
-    case 4: k_contract_tiles<Cfg16x128><<<grid, Cfg16x128::kThreads, 0, s>>>(g); break;
-    default: k_contract_tiles<Cfg32x32><<<grid, Cfg32x32::kThreads, 0, s>>>(g); break;
-  }
-  SHT_CUDA(cudaGetLastError());
-}
 
 // The FP64 tiles of a split plan's work list, computed only when the device word *flag is set
 // (an operand of the execute holds a non-finite value): persistent, one 128 x 32 tile per
@@ -328,31 +296,6 @@ static ModeMap make_modemap(const std::vector<int>& x, const std::vector<int>& y
   m.n = (int)x.size();
   for (size_t i = 0; i < x.size(); ++i) { m.x[i] = x[i]; m.y[i] = y[i]; }
   return m;
-}
-
-// median-ish tile choice for the plain path: the shape that wastes the least tile area
-// over the C blocks' (m, n), sampled from the host index
-static int choose_plain_shape(const sht_plan* p) {
-  const sht_tensor* C = p->C;
-  if (C->nblocks == 0) return 0;
-  const int stride = std::max<int64_t>(1, C->nblocks / 512);
-  double best = 1e300;
-  int best_i = 0;
-  for (int si = 0; si < kNumShapes; ++si) {
-    double waste = 0;
-    for (int64_t b = 0; b < C->nblocks; b += stride) {
-      const int64_t id = C->ids[b];
-      int64_t m = 1, n = 1;
-      for (int ax : p->maps.rowC) m *= C->bs[ax][(id / C->gstride[ax]) % C->nblk[ax]];
-      for (int ax : p->maps.colC) n *= C->bs[ax][(id / C->gstride[ax]) % C->nblk[ax]];
-      const int64_t tm = kShapes[si].tm, tn = kShapes[si].tn;
-      const double area = (double)((m + tm - 1) / tm * tm) * (double)((n + tn - 1) / tn * tn);
-      // padded area plus a per-tile fixed cost of 2k elements
-      waste += area + 2048.0 * (double)(((m + tm - 1) / tm) * ((n + tn - 1) / tn));
-    }
-    if (waste < best) { best = waste; best_i = si; }
-  }
-  return best_i;
 }
 
 // per C block: matrix extents m, n, the sum over its pairs of the contracted extent, flops
@@ -457,7 +400,6 @@ void plan_build(sht_plan* p, cudaStream_t s, bool speculate) {
   for (sht_tensor* t : {A, B, C}) tensor_touch(t, s);
   const double eps = p->eps;
   const sht_norm norm = p->norm;
-  const sht_mode mode = p->mode;
   const ShtMaps& mp = p->maps;
   DevicePool* pool = ctx->pool.get();
   const long long nA = A->nblocks, nB = B->nblocks;
@@ -578,8 +520,11 @@ void plan_build(sht_plan* p, cudaStream_t s, bool speculate) {
       }
       p->d_pair_a = PoolBuf(pool, np * 4, s);
       p->d_pair_b = PoolBuf(pool, np * 4, s);
-      k_gather_pairs<<<grid_for(np, 256), 256, 0, s>>>(porder.as<int>(), pa.as<int>(), pb.as<int>(), np,
-                                                        p->d_pair_a.as<int>(), p->d_pair_b.as<int>());
+      if (p->mode != SHT_MODE_SPLIT) p->d_recs = PoolBuf(pool, np * sizeof(PairRec), s);
+      k_gather_pairs<<<grid_for(np, 256), 256, 0, s>>>(
+          porder.as<int>(), pa.as<int>(), pb.as<int>(), np, p->d_pair_a.as<int>(), p->d_pair_b.as<int>(),
+          p->d_recs.as<PairRec>(), rec_modes(A->order, mp.rowA, mp.colA), rec_modes(B->order, mp.colB, mp.rowB),
+          A->d_offsets.as<long long>(), A->d_dims.as<int>(), B->d_offsets.as<long long>(), B->d_dims.as<int>());
       SHT_CUDA(cudaGetLastError());
     }
   }
@@ -694,48 +639,7 @@ void plan_build(sht_plan* p, cudaStream_t s, bool speculate) {
   // per C block m, n, sum of the pairs' k and flops; the total flop count
   cblock_stats(p, s);
   trace("plan: pstart+flops", s);
-  if (mode == SHT_MODE_PLAIN_FP64) {
-    p->shape = choose_plain_shape(p);
-    build_work(p, kShapes[p->shape].tm, kShapes[p->shape].tn, s);
-    trace("plan: plain work list", s);
-  }
   p->plan_ms += now_ms() - t0;
-}
-
-void build_work(sht_plan* p, int TM, int TN, cudaStream_t s) {
-  DevicePool* pool = p->ctx->pool.get();
-  const long long nc = p->ncblk;
-  p->nwork = p->nwork_touched = 0;
-  if (nc == 0) return;
-  PoolBuf ct(pool, nc * 8, s), cu(pool, nc * 8, s), ot(pool, nc * 8, s), ou(pool, nc * 8, s);
-  k_tile_counts<<<grid_for(nc, 256), 256, 0, s>>>(p->C->d_dims.as<int>(), p->C->order, p->tmaps.row, p->tmaps.col, nc,
-                                                   p->d_pstart.as<int>(), TM, TN, ct.as<long long>(), cu.as<long long>());
-  SHT_CUDA(cudaGetLastError());
-  size_t tb = 0;
-  cub::DeviceScan::ExclusiveSum(nullptr, tb, ct.as<long long>(), ot.as<long long>(), (int)nc, s);
-  {
-    PoolBuf tmp(pool, tb, s);
-    cub::DeviceScan::ExclusiveSum(tmp.ptr, tb, ct.as<long long>(), ot.as<long long>(), (int)nc, s);
-    cub::DeviceScan::ExclusiveSum(tmp.ptr, tb, cu.as<long long>(), ou.as<long long>(), (int)nc, s);
-  }
-  const long long nt = d2h_scalar<long long>(ot.as<long long>() + nc - 1, s) + d2h_scalar<long long>(ct.as<long long>() + nc - 1, s);
-  const long long nu = d2h_scalar<long long>(ou.as<long long>() + nc - 1, s) + d2h_scalar<long long>(cu.as<long long>() + nc - 1, s);
-  if (nt + nu > (long long)INT32_MAX) fail(SHT_ERR_UNSUPPORTED, "work list above 2^31 tiles");
-  p->d_work = PoolBuf(pool, std::max(nt + nu, 1LL) * 8, s);
-  k_tile_emit<<<grid_for(nc, 128), 128, 0, s>>>(nc, ct.as<long long>(), ot.as<long long>(), cu.as<long long>(),
-                                                 ou.as<long long>(), nt, p->d_work.as<int2>());
-  SHT_CUDA(cudaGetLastError());
-  plan_flops(p, s);  // the stream is idle after the reads above
-  if (p->d_npairs.ptr) {
-    // the pair list was sized from the host patterns: the device must have found as many
-    if (d2h_scalar<long long>(p->d_npairs.ptr, s) != p->npairs)
-      fail(SHT_ERR_STATE, "pair count of the host patterns differs from the device's");
-    p->d_npairs = PoolBuf();
-  }
-  p->nwork_touched = nt;
-  p->nwork = nt + nu;
-  p->work_tm = TM;
-  p->work_tn = TN;
 }
 
 SparseArgs sparse_args(sht_plan* p, double alpha, double beta) {
@@ -750,16 +654,13 @@ SparseArgs sparse_args(sht_plan* p, double alpha, double beta) {
   g.B = B->d_data.as<double>(); g.offB = B->d_offsets.as<long long>(); g.dimsB = B->d_dims.as<int>();
   g.C = C->d_data.as<double>(); g.offC = C->d_offsets.as<long long>(); g.dimsC = C->d_dims.as<int>();
   g.pair_a = p->d_pair_a.as<int>(); g.pair_b = p->d_pair_b.as<int>(); g.pstart = p->d_pstart.as<int>();
-  g.work = p->d_work.as<int2>();
+  g.recs = p->d_recs.as<PairRec>();
   return g;
 }
 
 void plan_touch(sht_plan* p, cudaStream_t s) {
   for (sht_tensor* t : {p->A, p->B, p->C}) tensor_touch(t, s);
-  for (PoolBuf* b : {&p->d_pair_a, &p->d_pair_b, &p->d_pstart, &p->d_work, &p->d_bwork, &p->d_counter, &p->mf_a,
-                     &p->mf_b, &p->mf_aoff, &p->mf_boff, &p->mf_ald, &p->mf_bld, &p->mf_ak4, &p->mf_aitems,
-                     &p->mf_bitems})
-    b->use_on(s);
+  for (PoolBuf* b : {&p->d_pair_a, &p->d_pair_b, &p->d_recs, &p->d_pstart, &p->d_bwork, &p->d_counter}) b->use_on(s);
   for (PoolBuf* b : {&p->sp_a, &p->sp_b, &p->sp_ae, &p->sp_be, &p->sp_bsc, &p->sp_meta, &p->sp_items, &p->sp_pairs,
                      &p->sp_rowtab, &p->sp_coltab})
     b->use_on(s);
@@ -768,19 +669,8 @@ void plan_touch(sht_plan* p, cudaStream_t s) {
 void plan_execute(sht_plan* p, double alpha, double beta, cudaStream_t s) {
   plan_touch(p, s);
   const SparseArgs g = sparse_args(p, alpha, beta);
-  uint64_t one;
-  const double d1 = 1.0;
-  std::memcpy(&one, &d1, 8);
-  uint64_t bb;
-  std::memcpy(&bb, &beta, 8);
-  const long long nwork = (bb == one) ? p->nwork_touched : p->nwork;
-  if (p->mode == SHT_MODE_BATCHED_FP64) {
-    batched_execute(p, g, nwork, s);
-  } else if (p->mode == SHT_MODE_SPLIT) {
-    split_execute(p, g, s);
-  } else {
-    launch_tiles(p->shape, nwork, g, s);
-  }
+  if (p->mode == SHT_MODE_SPLIT) split_execute(p, g, s);
+  else ring_launch(p, g, s);
 }
 
 }  // namespace sht

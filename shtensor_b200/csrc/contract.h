@@ -11,7 +11,7 @@ struct sht_plan {
   sht_tensor *A = nullptr, *B = nullptr, *C = nullptr;
   ShtMaps maps;
   sht::TileMaps tmaps{};
-  long long npairs = 0, ncblk = 0, nwork = 0, nwork_touched = 0;
+  long long npairs = 0, ncblk = 0;
   double flops = 0.0, plan_ms = 0.0, exec_ms = 0.0;
   double eps = 0.0;                 // screening threshold and norm of the pair list
   sht_norm norm = SHT_NORM_FROBENIUS;
@@ -20,25 +20,13 @@ struct sht_plan {
   sht::PoolBuf d_missing;           // product blocks absent from C, when the build assumed none
   bool flops_pending = false;       // d_flops not yet copied into flops
   cudaEvent_t flops_event = nullptr;  // recorded after d_flops is computed
-  int shape = 0, work_tm = 64, work_tn = 64;
   sht::PoolBuf d_pair_a, d_pair_b;  // int32 storage indices into A / B, canonical order
+  sht::PoolBuf d_recs;              // PairRec per pair (FP64 forms)
   sht::PoolBuf d_pstart;            // int32[ncblk + 1]
-  sht::PoolBuf d_work;              // int2 (C block, tile) for the plain path
   sht::PoolBuf d_cm, d_cn, d_cksum; // per C block: rows, columns, sum of the pairs' k
-  // batched path
-  sht::PoolBuf d_bwork;             // int4 (C block, tile, class, 0)
-  sht::PoolBuf d_counter;           // work counter of the persistent kernel
+  sht::PoolBuf d_bwork;             // int4 per tile (ring_item; split plans: (C block, tile, ., .))
+  sht::PoolBuf d_counter;           // work counter of the persistent FP64 kernel
   long long bwork = 0, bwork_touched = 0;
-  int bclass_shape[8] = {0};
-  int nclass = 0;
-  // matrix form of the operands (batched and split paths)
-  sht::PoolBuf mf_a, mf_b;          // A_mat / B_mat elements
-  sht::PoolBuf mf_aoff, mf_boff;    // int64 per block offsets
-  sht::PoolBuf mf_ald, mf_bld;      // int32 per block leading dimensions (even)
-  sht::PoolBuf mf_ak4;              // int32 per A block contracted extent rounded up to 4
-  sht::PoolBuf mf_aitems, mf_bitems;  // int4 (block, k0, k1, 0) slabs of the matform kernel
-  long long mf_naitems = 0, mf_nbitems = 0;
-  long long mf_elems = 0;
   // split path: INT8 slices (K-major rows), row / column exponents, error words
   sht::PoolBuf sp_a, sp_b, sp_ae, sp_be;
   sht::PoolBuf sp_bsc;                // B column scales 2^f as doubles (the reassembly's)
@@ -76,13 +64,13 @@ sht_plan* plan_init(sht_ctx* ctx, const std::string& expr, sht_tensor* A, sht_te
 // saves a synchronization when C is contracted into repeatedly.
 void plan_build(sht_plan* p, cudaStream_t s, bool speculate = false);
 struct PatternGrew {};
-void build_work(sht_plan* p, int TM, int TN, cudaStream_t s);
 void cblock_stats(sht_plan* p, cudaStream_t s);
 // The plan's flop count; the first call after planning copies it from the device (a sync),
 // so callers that synchronize anyway read it right after.
 double plan_flops(sht_plan* p, cudaStream_t s);
-// Cost-ordered work list (C block, tile, shape) on the device: fixed_shape >= 0 uses one
-// shape (tm x tn) for every block, otherwise per size class from class_shape (or the model).
+// Cost-ordered work list on the device.  fixed_tm > 0 (split plans): tiles of fixed_tm x fixed_tn, items
+// (C block, tile, ., .).  Otherwise the model's tile shape (tile_types.h) for every block, or with
+// per_class the autotuner's choice for the block's size class where there is one; items as ring_item.
 // A device scalar, or the sum of two (b may be null), for a read-back.
 struct DevSum {
   const long long* a;
@@ -95,12 +83,10 @@ void device_work_list(sht_plan* p, int fixed_tm, int fixed_tn, bool per_class, c
                       const DevSum* extra = nullptr, long long* extra_out = nullptr, int nextra = 0,
                       const unsigned long long* order_key = nullptr, int order_bits = 0);
 void plan_execute(sht_plan* p, double alpha, double beta, cudaStream_t s);
-void batched_prepare(sht_plan* p, cudaStream_t s);
-// the persistent kernel alone, with the operands already in matrix form (matform_execute)
-void batched_launch(sht_plan* p, const SparseArgs& g, cudaStream_t s);
-void batched_execute(sht_plan* p, const SparseArgs& g, long long nwork_plain, cudaStream_t s);
+// the FP64 forms: work list and counter, then the persistent kernel
+void ring_prepare(sht_plan* p, cudaStream_t s);
+void ring_launch(sht_plan* p, const SparseArgs& g, cudaStream_t s);
 void autotune(sht_plan* p, const char* cache_file, cudaStream_t s);
-void matform_prepare(sht_plan* p, cudaStream_t s);
 size_t batched_desc_bytes();
 int batched_ctas_per_sm(sht_ctx* ctx);
 long long batched_multi_launch(sht_ctx* ctx, const std::vector<sht_plan*>& plans, const std::vector<SparseArgs>& args,
@@ -130,7 +116,6 @@ size_t split_desc_bytes();
 bool split_flags_clear(sht_plan* p, cudaStream_t s);
 long long split_multi_launch(sht_ctx* ctx, const std::vector<sht_plan*>& plans, const std::vector<SparseArgs>& args,
                              void* host_descs, PoolBuf& descs, cudaStream_t s);
-void matform_execute(sht_plan* p, double alpha, cudaStream_t s);
 void block_dims_sizes(const sht_tensor* t, const long long* ids, long long n, int* dims, long long* sizes,
                       cudaStream_t s);
 void tensor_compress_device(sht_tensor* t, cudaStream_t s);

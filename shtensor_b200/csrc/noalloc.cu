@@ -57,7 +57,7 @@ struct StackForm {
   double kpad;
 };
 
-// one CTA per op: the op's block into matrix form (as k_matform does for block-sparse plans)
+// one CTA per op: the op's block into matrix form
 __global__ void __launch_bounds__(256) k_matform_stack(const double* __restrict__ src, StackForm f,
                                                        double* __restrict__ dst, long long nb_ops) {
   int st[kMaxOrder];

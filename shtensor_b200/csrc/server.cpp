@@ -5,7 +5,7 @@
 // thread and `planners` planner threads.  A request moves through
 //   queued    submitted, waiting for a slot, for pool memory, or for an earlier request that
 //             touches the same tensor (the loop decides admission);
-//   planning  with a planner thread: matching, C pattern, work list and operands in matrix form
+//   planning  with a planner thread: matching, C pattern, work list
 //             on that planner's own stream, ending with an event;
 //   ready     planned, waiting for the next launch;
 //   running   in one of at most two persistent launches queued on the exec stream.
@@ -164,10 +164,12 @@ struct sht_server {
 namespace {
 
 
-// device bytes a request needs beyond its tensors, estimated before planning: the operands in
-// matrix form (batched: about 10 bytes per element with padding) or as slices (split: S bytes
-// per element of rows padded to the tile height and k to 32, about 24 at S = 7), plus pair,
-// work and C-pattern arrays (C's own growth is not known until matching)
+// Device bytes admission counts for a request beyond its tensors, before planning: in the split form
+// the slices (S bytes per element of rows padded to the tile height and k to 32, about 24 at S = 7);
+// in the batched form, whose kernel reads the operands in place, 10 bytes per operand element all the
+// same, so that the pool's room bounds how many large requests are in flight as it did when each
+// held a copy of its operands; plus pair, work and C-pattern arrays (C's own growth is not known
+// until matching).
 size_t estimate_bytes(const Request& r, int mode) {
   const double elems = (double)r.A->nnz + (double)r.B->nnz;
   const double blocks = (double)r.A->nblocks + (double)r.B->nblocks + (double)r.C->nblocks;
@@ -313,6 +315,11 @@ bool sht_server::admit() {
     // requests with the planners may not have taken their memory yet: count their estimates
     size_t planning_bytes = 0;
     for (const ReqPtr& o : planning) planning_bytes += estimate_bytes(*o, mode);
+    // planned batched-form requests hold no scratch of that size: their estimates count on
+    auto count_on = [&](const Request& o) { return o.kind < 0 ? estimate_bytes(o, SHT_MODE_BATCHED_FP64) : 0; };
+    for (const ReqPtr& o : ready) planning_bytes += count_on(*o);
+    for (const auto& l : running)
+      for (const ReqPtr& o : l->reqs) planning_bytes += count_on(*o);
     const size_t free_now = ctx->pool->free_bytes();
     const size_t avail = free_now > planning_bytes ? free_now - planning_bytes : 0;
     if (others && avail < reserve_bytes + estimate_bytes(r, mode)) {
@@ -389,9 +396,7 @@ void sht_server::planner(int index) {
         r->form = SHT_MODE_BATCHED_FP64;
         r->kind = -1;
         r->plan.reset(sht::plan_create(ctx, r->expr, r->A, r->B, r->C, r->eps, r->norm, SHT_MODE_BATCHED_FP64, s));
-        sht::batched_prepare(r->plan.get(), s);
-        const sht::SparseArgs g = sht::sparse_args(r->plan.get(), r->alpha, r->beta);
-        if (!g.sc.alpha_zero) sht::matform_execute(r->plan.get(), r->alpha, s);
+        sht::ring_prepare(r->plan.get(), s);
       }
       SHT_CUDA(cudaEventRecord(r->planned, s));
       r->npairs = r->plan->npairs;

@@ -51,6 +51,7 @@
 
 #include "contract.h"
 #include "device_common.cuh"
+#include "mbar.cuh"
 #include "tile_core.cuh"
 
 namespace sht {
@@ -427,8 +428,6 @@ static const SliceKernel kSliceKernels[kMaxSlices] = {k_slice<1>, k_slice<2>, k_
                                                       k_slice<5>, k_slice<6>, k_slice<7>, k_slice<8>};
 
 // ------------------------------------------------------------------ tcgen05 helpers
-__device__ __forceinline__ unsigned smem_u32(const void* p) { return static_cast<unsigned>(__cvta_generic_to_shared(p)); }
-
 // K-major, no swizzle: core matrices of 8 rows x 16 bytes; LBO = 128 (the two 16-byte halves
 // of a 32-byte K step), SBO = 256 (next 8 rows).
 __device__ __forceinline__ unsigned long long umma_desc(const void* smem) {
@@ -456,10 +455,6 @@ __device__ __forceinline__ void umma_commit(void* mbar) {
                : "memory");
 }
 
-__device__ __forceinline__ void mbar_init(void* mbar, unsigned count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(mbar)), "r"(count) : "memory");
-}
-
 __device__ __forceinline__ void tmem_ld16(unsigned taddr, unsigned* v) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
@@ -485,22 +480,6 @@ __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence:
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
 // ------------------------------------------------------------------ mbarrier / bulk copies
-__device__ __forceinline__ bool mbar_try(void* mbar, unsigned parity) {
-  unsigned ok;
-  asm volatile(
-      "{\n\t.reg .pred P;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 P, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, P;\n\t}\n"
-      : "=r"(ok)
-      : "r"(smem_u32(mbar)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-
-__device__ __forceinline__ void mbar_arrive(void* mbar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(mbar)) : "memory");
-}
-
 __device__ __forceinline__ void mbar_expect_tx(void* mbar, unsigned bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(mbar)), "r"(bytes) : "memory");
 }
@@ -787,14 +766,7 @@ __device__ __forceinline__ SplitReq split_req(const SplitArgs& g, int item, int&
 
 // bounded wait that also gives up when another role raised the abort flag
 __device__ __forceinline__ bool split_wait(void* mbar, unsigned parity, volatile int* abort, const SplitArgs& g) {
-  for (long long i = 0; i < g.wait_limit; ++i) {
-    if (mbar_try(mbar, parity)) return true;
-    if (*abort) return false;
-  }
-  *abort = 1;
-  *g.err = (int)SHT_ERR_TIMEOUT;  // every writer stores the same value
-  __threadfence_system();
-  return false;
+  return mbar_wait_bounded(mbar, parity, abort, g.wait_limit, g.err);
 }
 
 // bounded wait for work this CTA issued already (bulk copies, MMAs): it always completes, so

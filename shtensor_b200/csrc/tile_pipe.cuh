@@ -1,4 +1,5 @@
-// tile_pipe.cuh -- pipelined output-stationary FP64 tile on the FP64 tensor cores (batched form).
+// tile_pipe.cuh -- pipelined output-stationary FP64 tile on the FP64 tensor cores, operands in matrix
+// form (the allocation-free stack call, noalloc.cu; tile_ring.cuh is the tile of the other calls).
 //
 // Arithmetic per output element is the reference XMM kernel's (src/Kernel/KernelImpl.cpp:
 // 594-619, 661-683): c = beta*c (0 when beta is +0.0), then for every pair in order and every
@@ -9,7 +10,7 @@
 // length is not a multiple of 4 is padded with a = -0.0, b = +0.0: fma(-0, +0, c) == c for
 // every c, signed zeros included.
 //
-// Operands come in matrix form (matform.cu): every A block as an m_pad x K4 column-major
+// Operands come in matrix form (written by noalloc.cu's first pass): every A block as an m_pad x K4 column-major
 // matrix with alpha applied and the K padding set to -0.0, every B block as an n_pad x K4
 // matrix (columns fastest) with +0.0 padding, m_pad/n_pad even and each block 16-byte
 // aligned.  So:

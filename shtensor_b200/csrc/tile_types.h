@@ -26,6 +26,31 @@ struct TileScalars {
   int alpha_zero;  // alpha is +0.0: products skipped
 };
 
+// Tile shapes of the FP64 kernel: the most rows and columns of a tile (at most 64 each).
+constexpr int kRingShapes = 4;
+__host__ __device__ constexpr int ring_tm(int s) { return s & 2 ? 32 : 64; }
+__host__ __device__ constexpr int ring_tn(int s) { return s & 1 ? 32 : 64; }
+// number of tiles along an extent, and their size (the last tile may be smaller)
+__host__ __device__ __forceinline__ int ring_ntiles(int ext, int t) { return (ext + t - 1) / t; }
+__host__ __device__ __forceinline__ int ring_step(int ext, int nt) { return (((ext + nt - 1) / nt) + 7) & ~7; }
+
+// One block pair of a plan as the FP64 kernel reads it: where its blocks start, the contracted extent
+// and the strides of linear addressing (tile_ring.cuh).  Built once per pair; every tile of the pair's
+// C block reads it.
+struct PairRec {
+  long long offA, offB;
+  int K, rsA, ksA, rsB, ksB, ia, ib, pad;
+};
+static_assert(sizeof(PairRec) == 48, "read in 16-byte units");
+
+// One tile of a work list: C block, first row and column, rows | columns << 16.
+__host__ __device__ __forceinline__ int4 ring_item(int c, int tile, int m, int n, int tm, int tn) {
+  const int ntr = ring_ntiles(m, tm), sr = ring_step(m, ntr), sc = ring_step(n, ring_ntiles(n, tn));
+  const int r0 = tile % ntr * sr, c0 = tile / ntr * sc;
+  const int mt = m - r0 < sr ? m - r0 : sr, nt = n - c0 < sc ? n - c0 : sc;
+  return make_int4(c, r0, c0, mt | nt << 16);
+}
+
 // Device pointers and scalars of one block-sparse execute (plain and batched forms).
 struct SparseArgs {
   TileMaps mp;
@@ -34,7 +59,7 @@ struct SparseArgs {
   const double* B; const long long* offB; const int* dimsB;
   double* C; const long long* offC; const int* dimsC;
   const int* pair_a; const int* pair_b; const int* pstart;
-  const int2* work;
+  const PairRec* recs;  // the FP64 forms (null in a split plan)
 };
 
 }  // namespace sht
