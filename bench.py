@@ -568,14 +568,16 @@ def run_reference(args):
     rank, world, _ = dist_env()
     if rank != 0:
         return
+    import oracle
+    ref = oracle.ref_lib() is not None  # without the reference's sources: the restatement, as "port"
     nthreads = os.cpu_count() or 1
     w = build_workload(args.workload, args.seed, args.scale)
     vals = []
     leg = None
     for _ in range(args.warmup):
-        cpu_leg(w, max(args.cpu_sample_seconds / 5, 1.0), nthreads, True, 1)
+        cpu_leg(w, max(args.cpu_sample_seconds / 5, 1.0), nthreads, ref, 1)
     for _ in range(args.steps):
-        leg = cpu_leg(w, args.cpu_sample_seconds / max(args.steps, 1), nthreads, True, 1)
+        leg = cpu_leg(w, args.cpu_sample_seconds / max(args.steps, 1), nthreads, ref, 1)
         vals.append(leg["value"])
     value = float(np.median(vals))
     line = {
@@ -583,7 +585,7 @@ def run_reference(args):
         "steps": args.steps, "warmup": args.warmup, "higher_is_better": True, "scaling": "weak",
         "vs_baseline": None, "dtype": "f64", "data": "synthetic (seeded)",
         "config": {"workload": WORKLOADS[args.workload], "scale": args.scale, "seed": args.seed},
-        "cpu_baseline": {"value": value, "unit": "GFLOP/s", "cores": nthreads, "kind": "reference",
+        "cpu_baseline": {"value": value, "unit": "GFLOP/s", "cores": nthreads, "kind": leg["kind"],
                          "sample": leg["sample"]},
         "e2e": {"value": value, "unit": "GFLOP/s", "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 0},
     }
