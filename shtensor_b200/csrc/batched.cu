@@ -413,6 +413,31 @@ long long batched_multi_launch(sht_ctx* ctx, const std::vector<sht_plan*>& plans
   return total;
 }
 
+void ring_stack(sht_ctx* ctx, const SparseArgs& a, const PairRec& rec, const int* dA, const int* dB, const int* dC,
+                long long size_a, long long size_b, long long size_c, int m, int n, long long nb_ops, cudaStream_t s) {
+  RingArgs r{};
+  r.mp = a.mp;
+  r.sc = a.sc;
+  r.flags = ring_flags(a.mp, a.A, a.B);
+  r.A = a.A; r.B = a.B; r.C = a.C;
+  r.stack = rec;
+  r.size_a = size_a; r.size_b = size_b; r.size_c = size_c;
+  std::copy(dA, dA + kMaxOrder, r.sdA);
+  std::copy(dB, dB + kMaxOrder, r.sdB);
+  std::copy(dC, dC + kMaxOrder, r.sdC);
+  r.m = m;
+  r.n = n;
+  const long long tiles = (long long)ring_ntiles(m, kRingTile) * ring_ntiles(n, kRingTile);
+  if (tiles * nb_ops > 0x7fffffffLL) fail(SHT_ERR_UNSUPPORTED, "stack too large for one launch");
+  r.tiles_per_op = (int)tiles;
+  r.nwork = (int)(tiles * nb_ops);
+  r.err = ctx_error_word(ctx);
+  r.wait_limit = kRingWaitLimit;
+  const int grid = std::min(ring_grid(ctx), r.nwork);
+  k_tiles<kRingStack><<<grid, kRingThreads, sizeof(RingSmem), s>>>(r);
+  SHT_CUDA(cudaGetLastError());
+}
+
 void ring_launch(sht_plan* p, const SparseArgs& g, cudaStream_t s) {
   launch_plan(p->ctx, ring_args(p, g), s);
   trace("tile kernel", s);

@@ -268,6 +268,7 @@ sht_status sht_kernel_create(sht_ctx* ctx, const char* expr, const int* sa, int 
     k->size_b = std::accumulate(k->sb.begin(), k->sb.end(), (int64_t)1, std::multiplies<int64_t>());
     k->size_c = std::accumulate(k->sc.begin(), k->sc.end(), (int64_t)1, std::multiplies<int64_t>());
     need(k->size_a < (1LL << 31) && k->size_b < (1LL << 31) && k->size_c < (1LL << 31), "block above 2^31 elements");
+    stack_prepare(k.get());
     *out = k.release();
   });
 }
@@ -275,6 +276,7 @@ sht_status sht_kernel_create(sht_ctx* ctx, const char* expr, const int* sa, int 
 sht_status sht_kernel_call(sht_kernel* k, const void* a, const void* b, void* c, int64_t nb_ops, void* stream) {
   return guard([&] {
     need(k, "null kernel");
+    raise_pending(k->ctx);
     stack_call(k, a, b, c, nb_ops, as_stream(stream));
   });
 }

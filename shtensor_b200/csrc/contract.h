@@ -86,6 +86,10 @@ void plan_execute(sht_plan* p, double alpha, double beta, cudaStream_t s);
 // the FP64 forms: work list and counter, then the persistent kernel
 void ring_prepare(sht_plan* p, cudaStream_t s);
 void ring_launch(sht_plan* p, const SparseArgs& g, cudaStream_t s);
+// a stack of equal block triples (Kernel<double>::call): one pair per C block, its extents and strides
+// in rec, its block extents in dA / dB / dC
+void ring_stack(sht_ctx* ctx, const SparseArgs& a, const PairRec& rec, const int* dA, const int* dB, const int* dC,
+                long long size_a, long long size_b, long long size_c, int m, int n, long long nb_ops, cudaStream_t s);
 void autotune(sht_plan* p, const char* cache_file, cudaStream_t s);
 size_t batched_desc_bytes();
 int batched_ctas_per_sm(sht_ctx* ctx);

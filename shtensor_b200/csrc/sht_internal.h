@@ -196,6 +196,7 @@ struct sht_kernel {
   sht_dtype dtype = SHT_F64;
   sht_kernel_type type = SHT_KERNEL_XMM;
   int64_t m = 0, n = 0, k = 0, size_a = 0, size_b = 0, size_c = 0;
+  bool swizzle = false;  // layout of the blocks staged in shared memory (stack_prepare)
 };
 
 struct sht_tensor {
@@ -250,6 +251,7 @@ void tensor_compare_device(sht_tensor* X, sht_tensor* R, double* max_abs, double
                            cudaStream_t s);
 
 // stack kernel (stack.cu)
+void stack_prepare(sht_kernel* k);
 void stack_call(sht_kernel* k, const void* a, const void* b, void* c, int64_t nb_ops,
                 cudaStream_t s);
 
