@@ -68,26 +68,6 @@ struct ClassKey {
   std::string str() const { return std::to_string(lm) + "," + std::to_string(ln) + "," + std::to_string(lk); }
 };
 
-// Cost of one C block per unit of contracted extent in a tile shape, in products: what the tensor
-// pipe runs (the tile's fragments of 8x8, and four times the busiest warp's, averaged: a tile
-// waits for its busiest warp, but another CTA fills the gap), the operand copies, and a fixed
-// cost per tile.
-__host__ __device__ static inline float shape_cost(int m, int n, int sh) {
-  const int ntr = ring_ntiles(m, ring_tm(sh)), ntc = ring_ntiles(n, ring_tn(sh));
-  const int fr = ring_step(m, ntr) / 8, fc = ring_step(n, ntc) / 8;
-  const float busiest = 4.0f * (float)(((fr + 1) / 2) * ((fc + 1) / 2));
-  return (float)ntr * (float)ntc * (32.0f * ((float)(fr * fc) + busiest) + 64.0f * (float)(fr + fc) + 512.0f);
-}
-__host__ __device__ static inline int model_shape(int m, int n) {
-  float best = 3.0e38f;
-  int bi = 0;
-  for (int s = 0; s < kRingShapes; ++s) {
-    const float c = shape_cost(m, n, s);
-    if (c < best) { best = c; bi = s; }
-  }
-  return bi;
-}
-
 struct HostPlanView {
   std::vector<long long> m, n, ksum;  // per C block
   std::vector<int> pstart;
@@ -181,12 +161,6 @@ static void launch_plan(sht_ctx* ctx, const RingArgs& g, cudaStream_t s) {
 }
 
 // ------------------------------------------------------------------ device work list
-__device__ __forceinline__ int ilog2ceil_dev(long long v) {
-  int b = 0;
-  while ((1LL << b) < v) ++b;
-  return b;
-}
-
 __global__ void k_block_shapes(const int* __restrict__ cm, const int* __restrict__ cn,
                                const long long* __restrict__ cksum, const int* __restrict__ pstart, long long nc,
                                const unsigned char* __restrict__ table, int fixed_tm, int fixed_tn,
@@ -198,12 +172,7 @@ __global__ void k_block_shapes(const int* __restrict__ cm, const int* __restrict
     const int np = pstart[c + 1] - pstart[c];
     int sh = 0;
     if (fixed_tm <= 0) {
-      int t = 255;
-      if (table) {
-        const int lm = min(ilog2ceil_dev(m), 31), ln = min(ilog2ceil_dev(n), 31);
-        const int lk = min(ilog2ceil_dev(np > 0 ? (ks / np > 0 ? ks / np : 1) : 1), 31);
-        t = table[(lm * 32 + ln) * 32 + lk];
-      }
+      const int t = table ? table[class_index((int)m, (int)n, np > 0 ? ks / np : 1)] : 255;
       sh = t != 255 ? t : model_shape((int)m, (int)n);
     }
     const long long tm = fixed_tm > 0 ? fixed_tm : ring_tm(sh), tn = fixed_tm > 0 ? fixed_tn : ring_tn(sh);
@@ -250,6 +219,19 @@ __global__ void k_collect(ScalarSrc src, long long* __restrict__ out) {
   if (i < src.n) out[i] = *src.v[i].a + (src.v[i].b ? *src.v[i].b : 0);
 }
 
+PoolBuf tuned_table(sht_ctx* ctx, cudaStream_t s) {
+  std::vector<unsigned char> h(32 * 32 * 32, 255);
+  for (auto& kv : ctx->tuned) {
+    int lm, ln, lk;
+    if (std::sscanf(kv.first.c_str(), "%d,%d,%d", &lm, &ln, &lk) == 3 && lm < 32 && ln < 32 && lk < 32)
+      h[(lm * 32 + ln) * 32 + lk] = (unsigned char)kv.second;
+  }
+  PoolBuf table(ctx->pool.get(), h.size(), s);
+  SHT_CUDA(cudaMemcpyAsync(table.ptr, h.data(), h.size(), cudaMemcpyHostToDevice, s));
+  SHT_CUDA(cudaStreamSynchronize(s));  // pageable source
+  return table;
+}
+
 void device_work_list(sht_plan* p, int fixed_tm, int fixed_tn, bool per_class, cudaStream_t s, const DevSum* extra,
                       long long* extra_out, int nextra, const unsigned long long* order_key, int order_bits) {
   if (nextra > 3) fail(SHT_ERR_INVALID, "work list: at most three extra scalars");
@@ -261,17 +243,7 @@ void device_work_list(sht_plan* p, int fixed_tm, int fixed_tn, bool per_class, c
     return;
   }
   PoolBuf table;
-  if (per_class && !p->ctx->tuned.empty()) {
-    std::vector<unsigned char> h(32 * 32 * 32, 255);
-    for (auto& kv : p->ctx->tuned) {
-      int lm, ln, lk;
-      if (std::sscanf(kv.first.c_str(), "%d,%d,%d", &lm, &ln, &lk) == 3 && lm < 32 && ln < 32 && lk < 32)
-        h[(lm * 32 + ln) * 32 + lk] = (unsigned char)kv.second;
-    }
-    table = PoolBuf(pool, h.size(), s);
-    SHT_CUDA(cudaMemcpyAsync(table.ptr, h.data(), h.size(), cudaMemcpyHostToDevice, s));
-    SHT_CUDA(cudaStreamSynchronize(s));  // pageable source
-  }
+  if (per_class && !p->ctx->tuned.empty()) table = tuned_table(p->ctx, s);
   PoolBuf shape(pool, nc * 4, s), tiles(pool, nc * 8, s), ttiles(pool, nc * 8, s), key(pool, nc * 8, s),
       idx(pool, nc * 4, s), key2(pool, nc * 8, s), idx2(pool, nc * 4, s), tsorted(pool, nc * 8, s),
       off(pool, nc * 8, s), sums(pool, 16, s);
@@ -346,8 +318,10 @@ void device_work_list(sht_plan* p, int fixed_tm, int fixed_tn, bool per_class, c
 }
 
 void ring_prepare(sht_plan* p, cudaStream_t s) {
-  p->d_counter = PoolBuf(p->ctx->pool.get(), 256, s);
-  device_work_list(p, 0, 0, p->mode == SHT_MODE_BATCHED_FP64, s);
+  if (!p->work_ready) {  // else it came with the pairs
+    p->d_counter = PoolBuf(p->ctx->pool.get(), 256, s);
+    device_work_list(p, 0, 0, p->mode == SHT_MODE_BATCHED_FP64, s);
+  }
   trace("work list", s);
 }
 

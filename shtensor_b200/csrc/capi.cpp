@@ -53,6 +53,9 @@ static void contract_split(sht_plan* p, double alpha, double beta, cudaStream_t 
   LaneLease lane(ctx);
   const cudaStream_t ps = lane.lane.stream;
   SHT_CUDA(cudaEventRecord(lane.lane.start, s));
+  p->caller_event = lane.lane.start;
+  // without screening the counting kernel of the plan goes ahead of the slicer, whose CTAs fill the SMs
+  if (!(p->eps > 0.0)) plan_match_begin(p, ps);
   split_layout(p, ctx->split_slices ? ctx->split_slices : split_slices_default(), s);
   split_slice(p, alpha, s);
   trace("contract: slicer launched", s);
@@ -76,6 +79,7 @@ static void contract_split(sht_plan* p, double alpha, double beta, cudaStream_t 
   plan_touch(p, s);
   split_launch(p, sparse_args(p, alpha, beta), s);
   trace("contract: split kernel launched", s);
+  plan_settle(p, ps);
 }
 
 // A bounded wait of an earlier launch on this context ran out: report it at this call.
@@ -99,6 +103,7 @@ static void contract_fp64(sht_plan* p, double alpha, double beta, cudaStream_t s
   LaneLease lane(ctx);
   const cudaStream_t ps = lane.lane.stream;
   SHT_CUDA(cudaEventRecord(lane.lane.start, s));
+  p->caller_event = lane.lane.start;
   if (p->eps > 0.0) SHT_CUDA(cudaStreamWaitEvent(ps, lane.lane.start, 0));
   try {
     plan_build(p, ps, true);
@@ -115,6 +120,7 @@ static void contract_fp64(sht_plan* p, double alpha, double beta, cudaStream_t s
   plan_touch(p, s);
   ring_launch(p, sparse_args(p, alpha, beta), s);
   trace("contract: tile kernel launched", s);
+  plan_settle(p, ps);
 }
 
 volatile int* ctx_error_word(sht_ctx* ctx) {
@@ -187,6 +193,7 @@ sht_status sht_finalize(sht_ctx* ctx) {
     cudaDeviceSynchronize();
     if (ctx->stage_stream) cudaStreamDestroy(ctx->stage_stream);
     if (ctx->err_host) cudaFreeHost(ctx->err_host);
+    for (void* h : ctx->pin_pages) cudaFreeHost(h);
     for (auto& l : ctx->lanes) {
       cudaEventDestroy(l.start);
       cudaEventDestroy(l.done);
@@ -575,6 +582,9 @@ sht_status sht_contract(sht_ctx* ctx, const char* expr, double alpha, sht_tensor
     std::unique_ptr<sht_plan> p;
     raise_pending(ctx);
     p.reset(plan_init(ctx, expr, A, B, C, eps, norm, mode, s));
+    uint64_t bits;
+    std::memcpy(&bits, &beta, 8);
+    p->c_overwritten = bits == 0;  // beta is +0.0: the kernels write every element of C and read none
     if (mode == SHT_MODE_SPLIT) contract_split(p.get(), alpha, beta, s);
     else contract_fp64(p.get(), alpha, beta, s);
     if (rep) {

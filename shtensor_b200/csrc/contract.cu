@@ -1,7 +1,9 @@
 // contract.cu -- block-sparse contraction on one GPU: the device plan.
 //
 // Plan (all on the device; the reference has no block-sparse contract, src/Tensor/Tensor.cpp
-// is empty, so the rules below are this library's canonical ones, restated in the oracle):
+// is empty, so the rules below are this library's canonical ones, restated in the oracle; the
+// steps are those of the general path, plans over small block grids reach the same lists without
+// sorts, see k_match):
 //   1. keys: per A block the rolled block indices of its contracted modes, per B block the
 //      same over B's contracted modes; the C id splits into an A part and a B part;
 //   2. B is radix-sorted by key (stable, so equal keys keep id order); every A block finds
@@ -152,6 +154,21 @@ __device__ __forceinline__ void rec_strides(const int* __restrict__ d, const Rec
   }
 }
 
+__device__ __forceinline__ PairRec pair_rec(int ia, int ib, const RecModes& ma, const RecModes& mb,
+                                            const long long* __restrict__ offA, const int* __restrict__ dimsA,
+                                            const long long* __restrict__ offB, const int* __restrict__ dimsB) {
+  PairRec r;
+  int kb;
+  r.offA = offA[ia];
+  r.offB = offB[ib];
+  rec_strides(dimsA + (long long)ia * ma.order, ma, r.rsA, r.ksA, r.K);
+  rec_strides(dimsB + (long long)ib * mb.order, mb, r.rsB, r.ksB, kb);
+  r.ia = ia;
+  r.ib = ib;
+  r.pad = 0;
+  return r;
+}
+
 // The pairs in canonical order, with their records when rec is given.
 __global__ void k_gather_pairs(const int* __restrict__ order, const int* __restrict__ pa_in, const int* __restrict__ pb_in,
                                long long n, int* __restrict__ pa, int* __restrict__ pb, PairRec* __restrict__ rec,
@@ -163,17 +180,7 @@ __global__ void k_gather_pairs(const int* __restrict__ order, const int* __restr
     const int ia = pa_in[o], ib = pb_in[o];
     pa[i] = ia;
     pb[i] = ib;
-    if (!rec) continue;
-    PairRec r;
-    int kb;
-    r.offA = offA[ia];
-    r.offB = offB[ib];
-    rec_strides(dimsA + (long long)ia * ma.order, ma, r.rsA, r.ksA, r.K);
-    rec_strides(dimsB + (long long)ib * mb.order, mb, r.rsB, r.ksB, kb);
-    r.ia = ia;
-    r.ib = ib;
-    r.pad = 0;
-    rec[i] = r;
+    if (rec) rec[i] = pair_rec(ia, ib, ma, mb, offA, dimsA, offB, dimsB);
   }
 }
 
@@ -258,6 +265,343 @@ __global__ void k_count_missing(const long long* __restrict__ pc, long long np, 
     if (lo == nc || cids[lo] != id) ++n;
   }
   if (n) atomicAdd(missing, n);
+}
+
+// ---------------------------------------------------------------------------------------
+// plans over small block grids (cluster-built)
+// ---------------------------------------------------------------------------------------
+// When C's block grid and the contracted block grid are small, the plan needs no sorts: C's cells
+// (block grid positions, in id order) are counted directly, and the pairs of one cell, which differ
+// in their contracted coordinates and so in their A block, are ranked by A block.  One cluster of
+// eight CTAs (k_match: hardware barriers, eight SMs) counts pairs, finds the result pattern and sums
+// what the host needs for its allocations; after one read-back, k_match_cells and k_match_pairs
+// write the pattern, the pairs and the work list.  The general path below takes about 45 launches
+// and reads for the same plan, two to five microseconds each: ijl,lk->ijk over 20 blocks per mode
+// (12,872 pairs), see the figures at match_build.
+constexpr int kMatchCtas = 8, kMatchThreads = 1024;
+constexpr long long kMatchCells = 1 << 18;  // C's block grid
+constexpr int kMatchKeys = 512;             // contracted block grid: also the most pairs of one cell
+constexpr int kMatchBuckets = 65;           // cost classes of work items, heaviest first; last: untouched
+constexpr int kMatchSums = 7;               // pairs, blocks, elements, tiles touched / untouched, flops, new blocks
+
+struct MatchArgs {
+  TensorMeta mA, mB, mC;
+  KeySpec ka, kb;
+  ModeMap row, col;
+  const long long *idsA, *idsB, *idsC;
+  long long nA, nB, nC;
+  const int* dimsA;
+  RecModes recA, recB;
+  const double *normA, *normB;  // null: no screening
+  double eps;
+  int ncell, kspan;
+  int tiles;                     // count tiles and order them (FP64 forms)
+  const unsigned char* table;    // the autotuner's shapes (null: the model's)
+  // workspace
+  int *kcnt, *blist, *keyA, *cellA, *kA, *keyB, *cellB, *rankB;
+  int *ccnt, *cold, *cidx, *pofs;
+  long long *cks, *eofs, *csum;
+  unsigned long long *bucket, *bcur;
+  long long* out;                // kMatchSums totals, host-mapped
+};
+
+__device__ __forceinline__ void match_sync() {
+  __threadfence();
+  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+
+// extents, tile shape and cost class of one cell
+struct MatchCell {
+  int m, n, sh, nt, bucket;
+  long long elems;
+};
+__device__ __forceinline__ MatchCell match_cell(const MatchArgs& g, int cell, int np, long long ks) {
+  MatchCell c{1, 1, 0, 0, 0, 1};
+  for (int t = 0; t < g.row.n; ++t) {
+    const int y = g.row.y[t];
+    c.m *= g.mC.bsizes[g.mC.bstart[y] + cell / (int)g.mC.gstride[y] % g.mC.nblk[y]];
+  }
+  for (int t = 0; t < g.col.n; ++t) {
+    const int y = g.col.y[t];
+    c.n *= g.mC.bsizes[g.mC.bstart[y] + cell / (int)g.mC.gstride[y] % g.mC.nblk[y]];
+  }
+  c.elems = (long long)c.m * c.n;
+  if (g.tiles) {
+    int t = 255;
+    if (g.table) t = g.table[class_index(c.m, c.n, np > 0 ? ks / np : 1)];
+    c.sh = t != 255 ? t : model_shape(c.m, c.n);
+    const int ntr = ring_ntiles(c.m, ring_tm(c.sh)), ntc = ring_ntiles(c.n, ring_tn(c.sh));
+    c.nt = ntr * ntc;
+    // cost of a tile in half octaves, heaviest first
+    const float cost = (float)ring_step(c.m, ntr) * (float)ring_step(c.n, ntc) * (float)ks + 1.0f;
+    c.bucket = np > 0 ? kMatchBuckets - 2 - min(kMatchBuckets - 2, (int)(__float_as_uint(cost) >> 22) - 254)
+                      : kMatchBuckets - 1;
+  }
+  return c;
+}
+
+// inclusive scan over the CTA (1024 threads); scratch: 32 values
+template <typename T>
+__device__ __forceinline__ T match_scan(T v, T* scratch) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int d = 1; d < 32; d <<= 1) {
+    const T o = __shfl_up_sync(0xffffffffu, v, d);
+    if (lane >= d) v += o;
+  }
+  __syncthreads();
+  if (lane == 31) scratch[warp] = v;
+  __syncthreads();
+  if (warp == 0) {
+    T w = scratch[lane];
+    for (int d = 1; d < 32; d <<= 1) {
+      const T o = __shfl_up_sync(0xffffffffu, w, d);
+      if (lane >= d) w += o;
+    }
+    scratch[lane] = w;
+  }
+  __syncthreads();
+  return warp ? v + scratch[warp - 1] : v;
+}
+
+// the surviving pairs of A block a, a warp at a time: f(b, cell)
+template <class F>
+__device__ __forceinline__ void match_pairs_of(const MatchArgs& g, const int* kstart, int a, int lane, F f) {
+  const int k = g.keyA[a], cell = g.cellA[a];
+  const double na = g.normA ? g.normA[a] : 0.0;
+  for (int j = kstart[k] + lane; j < kstart[k + 1]; j += 32) {
+    const int b = g.blist[j];
+    if (g.normA && !(na * g.normB[b] >= g.eps)) continue;
+    f(b, cell + g.cellB[b]);
+  }
+}
+
+__device__ __forceinline__ void match_kstart(const MatchArgs& g, int* kstart) {
+  // exclusive starts of the contracted keys' B lists, per CTA (warp 0)
+  if (threadIdx.x < 32) {
+    int base = 0;
+    for (int i = 0; i < g.kspan; i += 32) {
+      const int l = threadIdx.x, v = i + l < g.kspan ? g.kcnt[i + l] : 0;
+      int x = v;
+      for (int d = 1; d < 32; d <<= 1) {
+        const int o = __shfl_up_sync(0xffffffffu, x, d);
+        if (l >= d) x += o;
+      }
+      if (i + l < g.kspan) kstart[i + l] = base + x - v;
+      base += __shfl_sync(0xffffffffu, x, 31);
+    }
+    if (threadIdx.x == 0) kstart[g.kspan] = base;
+  }
+  __syncthreads();
+}
+
+__global__ void __cluster_dims__(kMatchCtas, 1, 1) __launch_bounds__(kMatchThreads) k_match(const __grid_constant__ MatchArgs g) {
+  __shared__ int kstart[kMatchKeys + 1];
+  __shared__ long long scratch[32];
+  __shared__ int iscratch[32];
+  __shared__ unsigned long long hist[kMatchBuckets];
+  __shared__ long long sums[kMatchSums];
+  const int cta = blockIdx.x, gt = cta * kMatchThreads + threadIdx.x, nt = kMatchCtas * kMatchThreads;
+  const int lane = threadIdx.x & 31;
+  for (int i = gt; i < g.kspan; i += nt) g.kcnt[i] = 0;
+  for (int i = gt; i < g.ncell; i += nt) {
+    g.ccnt[i] = 0;
+    g.cold[i] = 0;
+    g.cks[i] = 0;
+  }
+  if (gt < kMatchBuckets) g.bucket[gt] = g.bcur[gt] = 0;
+  if (threadIdx.x < kMatchBuckets) hist[threadIdx.x] = 0;
+  if (threadIdx.x < kMatchSums) sums[threadIdx.x] = 0;
+  match_sync();
+  // keys and C parts of the operands' blocks; C's stored cells
+  for (int b = gt; b < g.nB; b += nt) {
+    int c[kMaxOrder];
+    unroll_block(g.mB, g.idsB[b], c);
+    long long k = 0, p = 0;
+    for (int t = 0; t < g.kb.nk; ++t) k += c[g.kb.kmode[t]] * g.kb.kstride[t];
+    for (int t = 0; t < g.kb.nf; ++t) p += c[g.kb.fmode[t]] * g.kb.fstride[t];
+    g.keyB[b] = (int)k;
+    g.cellB[b] = (int)p;
+    g.rankB[b] = atomicAdd(&g.kcnt[k], 1);
+  }
+  for (int a = gt; a < g.nA; a += nt) {
+    int c[kMaxOrder];
+    unroll_block(g.mA, g.idsA[a], c);
+    long long k = 0, p = 0;
+    int K = 1;
+    for (int t = 0; t < g.ka.nk; ++t) {
+      const int x = c[g.ka.kmode[t]];
+      k += x * g.ka.kstride[t];
+      K *= g.mA.bsizes[g.mA.bstart[g.ka.kmode[t]] + x];
+    }
+    for (int t = 0; t < g.ka.nf; ++t) p += c[g.ka.fmode[t]] * g.ka.fstride[t];
+    g.keyA[a] = (int)k;
+    g.cellA[a] = (int)p;
+    g.kA[a] = K;
+  }
+  for (int c = gt; c < g.nC; c += nt) g.cold[g.idsC[c]] = 1;
+  match_sync();
+  match_kstart(g, kstart);
+  for (int b = gt; b < g.nB; b += nt) g.blist[kstart[g.keyB[b]] + g.rankB[b]] = b;
+  match_sync();
+  // pairs per cell and their contracted extents
+  for (int a = gt >> 5; a < g.nA; a += nt >> 5)
+    match_pairs_of(g, kstart, a, lane, [&](int, int cell) {
+      atomicAdd(&g.ccnt[cell], 1);
+      atomicAdd(reinterpret_cast<unsigned long long*>(&g.cks[cell]), (unsigned long long)g.kA[a]);
+    });
+  match_sync();
+  // totals of this CTA's range of cells, and the cost classes
+  const int per = (g.ncell + kMatchCtas - 1) / kMatchCtas, c0 = min(g.ncell, cta * per), c1 = min(g.ncell, c0 + per);
+  {
+    long long v[kMatchSums] = {0, 0, 0, 0, 0, 0, 0};
+    for (int cell = c0 + threadIdx.x; cell < c1; cell += kMatchThreads) {
+      const int np = g.ccnt[cell], old = g.cold[cell];
+      if (!np && !old) continue;
+      const long long ks = g.cks[cell];
+      const MatchCell c = match_cell(g, cell, np, ks);
+      v[0] += np;
+      v[1] += 1;
+      v[2] += c.elems;
+      v[np ? 3 : 4] += c.nt;
+      v[5] += 2 * c.elems * ks;
+      v[6] += old ? 0 : 1;
+      if (g.tiles) atomicAdd(&hist[c.bucket], (unsigned long long)c.nt);
+    }
+#pragma unroll
+    for (int i = 0; i < kMatchSums; ++i) {
+      for (int d = 16; d; d >>= 1) v[i] += __shfl_xor_sync(0xffffffffu, v[i], d);
+      if (lane == 0 && v[i]) atomicAdd(reinterpret_cast<unsigned long long*>(&sums[i]), (unsigned long long)v[i]);
+    }
+    __syncthreads();
+    if (threadIdx.x < kMatchSums) g.csum[cta * kMatchSums + threadIdx.x] = sums[threadIdx.x];
+    if (threadIdx.x < kMatchBuckets && hist[threadIdx.x]) atomicAdd(&g.bucket[threadIdx.x], hist[threadIdx.x]);
+  }
+  match_sync();
+  // positions: pairs before each cell, its block number, its first element
+  long long base[3] = {0, 0, 0};
+  for (int r = 0; r < cta; ++r)
+    for (int i = 0; i < 3; ++i) base[i] += g.csum[r * kMatchSums + i];
+  for (int lo = c0; lo < c1; lo += kMatchThreads) {
+    const int cell = lo + threadIdx.x;
+    int np = 0, occ = 0;
+    long long el = 0;
+    if (cell < c1) {
+      np = g.ccnt[cell];
+      occ = np || g.cold[cell] ? 1 : 0;
+      if (occ) {
+        el = 1;
+        for (int d = 0; d < g.mC.order; ++d)
+          el *= g.mC.bsizes[g.mC.bstart[d] + cell / (int)g.mC.gstride[d] % g.mC.nblk[d]];
+      }
+    }
+    const int pi = match_scan(np, iscratch), oi = match_scan(occ, iscratch);
+    const long long ei = match_scan(el, scratch);
+    if (cell < c1) {
+      g.pofs[cell] = (int)base[0] + pi - np;
+      g.cidx[cell] = occ ? (int)base[1] + oi - 1 : -1;
+      g.eofs[cell] = base[2] + ei - el;
+    }
+    __syncthreads();
+    if (threadIdx.x == kMatchThreads - 1) {
+      sums[0] = pi;
+      sums[1] = oi;
+      sums[2] = ei;
+    }
+    __syncthreads();
+    for (int i = 0; i < 3; ++i) base[i] += sums[i];
+  }
+  if (cta == 0 && threadIdx.x < kMatchSums) {
+    long long v = 0;
+    for (int r = 0; r < kMatchCtas; ++r) v += g.csum[r * kMatchSums + threadIdx.x];
+    g.out[threadIdx.x] = v;
+    __threadfence_system();
+  }
+}
+
+// What k_match found, written into the plan's and (when the pattern grew) C's arrays.
+struct MatchOut {
+  int *pstart, *cm, *cn, *tmp_a, *tmp_b, *tmp_c;
+  long long* cksum;
+  long long *ids, *offs;  // C's new index (null: the pattern is unchanged)
+  int* dims;
+  int4* work;             // null: no work list
+  unsigned* counter;
+  long long npairs, nblocks;
+};
+__global__ void __launch_bounds__(256) k_match_cells(const __grid_constant__ MatchArgs g, MatchOut o) {
+  __shared__ int kstart[kMatchKeys + 1];
+  __shared__ unsigned long long bstart[kMatchBuckets];
+  match_kstart(g, kstart);
+  if (threadIdx.x == 0) {
+    unsigned long long s = 0;
+    for (int i = 0; i < kMatchBuckets; ++i) {
+      bstart[i] = s;
+      s += g.bucket[i];
+    }
+    if (blockIdx.x == 0) {
+      o.pstart[o.nblocks] = (int)o.npairs;
+      if (o.counter) *o.counter = 0;
+    }
+  }
+  __syncthreads();
+  const int lane = threadIdx.x & 31, gw = (blockIdx.x * 256 + threadIdx.x) >> 5, nw = gridDim.x * 8;
+  for (int base = gw * 32; base < g.ncell; base += nw * 32) {
+    const int cell = base + lane;
+    const int ci = cell < g.ncell ? g.cidx[cell] : -1;
+    MatchCell c{};
+    unsigned long long w0 = 0;
+    if (ci >= 0) {
+      const int np = g.ccnt[cell];
+      const long long ks = g.cks[cell];
+      c = match_cell(g, cell, np, ks);
+      o.pstart[ci] = g.pofs[cell];
+      o.cm[ci] = c.m;
+      o.cn[ci] = c.n;
+      o.cksum[ci] = ks;
+      if (o.ids) {
+        o.ids[ci] = cell;
+        o.offs[ci] = g.eofs[cell];
+        for (int d = 0; d < g.mC.order; ++d)
+          o.dims[(long long)ci * g.mC.order + d] =
+              g.mC.bsizes[g.mC.bstart[d] + cell / (int)g.mC.gstride[d] % g.mC.nblk[d]];
+      }
+      if (o.work) w0 = bstart[c.bucket] + atomicAdd(&g.bcur[c.bucket], (unsigned long long)c.nt);
+    }
+    // the cells' tiles, one cell after another, lanes over tiles
+    if (o.work)
+      for (unsigned todo = __ballot_sync(0xffffffffu, ci >= 0); todo; todo &= todo - 1) {
+        const int l = __ffs(todo) - 1;
+        const int m = __shfl_sync(0xffffffffu, c.m, l), n = __shfl_sync(0xffffffffu, c.n, l);
+        const int sh = __shfl_sync(0xffffffffu, c.sh, l), nt = __shfl_sync(0xffffffffu, c.nt, l);
+        const int cc = __shfl_sync(0xffffffffu, ci, l);
+        const unsigned long long w = __shfl_sync(0xffffffffu, w0, l);
+        for (int t = lane; t < nt; t += 32) o.work[w + t] = ring_item(cc, t, m, n, ring_tm(sh), ring_tn(sh));
+      }
+  }
+  for (int a = gw; a < g.nA; a += nw)
+    match_pairs_of(g, kstart, a, lane, [&](int b, int cell) {
+      // the old-block marks are not needed any more: the cells' cursors (from 0 or 1)
+      const int slot = g.pofs[cell] + (atomicAdd(&g.cold[cell], 2) >> 1);
+      o.tmp_a[slot] = a;
+      o.tmp_b[slot] = b;
+      o.tmp_c[slot] = g.cidx[cell];
+    });
+}
+
+// The pairs of each cell ranked by A block (no two have the same), with their records.
+__global__ void __launch_bounds__(256) k_match_pairs(MatchOut o, RecModes ma, RecModes mb, const long long* __restrict__ offA,
+                                                     const int* __restrict__ dimsA, const long long* __restrict__ offB,
+                                                     const int* __restrict__ dimsB, int* __restrict__ pa,
+                                                     int* __restrict__ pb, PairRec* __restrict__ rec) {
+  for (long long i = blockIdx.x * 256LL + threadIdx.x; i < o.npairs; i += gridDim.x * 256LL) {
+    const int a = o.tmp_a[i], b = o.tmp_b[i], c = o.tmp_c[i];
+    const int ps = o.pstart[c], pe = o.pstart[c + 1];
+    int rank = ps;
+    for (int q = ps; q < pe; ++q) rank += o.tmp_a[q] < a ? 1 : 0;
+    pa[rank] = a;
+    pb[rank] = b;
+    if (rec) rec[rank] = pair_rec(a, b, ma, mb, offA, dimsA, offB, dimsB);
+  }
 }
 
 // ---------------------------------------------------------------------------------------
@@ -355,10 +699,274 @@ double plan_flops(sht_plan* p, cudaStream_t s) {
   return p->flops;
 }
 
+// ------------------------------------------------------------------ plans over small block grids
+// A slot of host-mapped memory borrowed from the context for one plan's read-back.
+struct PinLease {
+  sht_ctx* ctx;
+  long long* host;
+  explicit PinLease(sht_ctx* c) : ctx(c) {
+    std::lock_guard<std::mutex> lk(ctx->lanes_mu);
+    if (ctx->pins.empty()) {
+      void* h = nullptr;
+      SHT_CUDA(cudaHostAlloc(&h, 4096, cudaHostAllocMapped));
+      ctx->pin_pages.push_back(h);
+      for (int i = 0; i < 32; ++i) ctx->pins.push_back(static_cast<long long*>(h) + 16 * i);
+    }
+    host = ctx->pins.back();
+    ctx->pins.pop_back();
+  }
+  ~PinLease() {
+    std::lock_guard<std::mutex> lk(ctx->lanes_mu);
+    ctx->pins.push_back(host);
+  }
+  PinLease(const PinLease&) = delete;
+  PinLease& operator=(const PinLease&) = delete;
+};
+
+struct MatchState {
+  MatchArgs g{};
+  PoolBuf ws, normA, normB, table;
+  PinLease pin;
+  cudaStream_t stream;
+  bool done = false;
+  explicit MatchState(sht_ctx* ctx, cudaStream_t s) : pin(ctx), stream(s) {}
+  // the kernel writes the pinned slot: it must have finished before the slot is lent again
+  ~MatchState() {
+    if (!done) cudaStreamSynchronize(stream);
+  }
+};
+
+}  // namespace sht
+
+sht_plan::~sht_plan() {
+  if (graph_exec) cudaGraphExecDestroy(graph_exec);
+  if (graph) cudaGraphDestroy(graph);
+  if (flops_event) cudaEventDestroy(flops_event);
+}
+sht_plan::sht_plan() = default;
+
+namespace sht {
+
+static void key_specs(const sht_plan* p, KeySpec& ka, KeySpec& kb, unsigned long long& kspan, long double& cgrid) {
+  const ShtMaps& mp = p->maps;
+  const sht_tensor *A = p->A, *C = p->C;
+  kspan = 1;
+  ka = KeySpec{};
+  kb = KeySpec{};
+  ka.nk = kb.nk = (int)mp.colA.size();
+  for (size_t t = 0; t < mp.colA.size(); ++t) {
+    ka.kmode[t] = mp.colA[t];
+    kb.kmode[t] = mp.rowB[t];
+    ka.kstride[t] = kb.kstride[t] = (long long)kspan;
+    const unsigned long long nb = (unsigned long long)A->nblk[mp.colA[t]];
+    if (kspan > (1ULL << 62) / nb) fail(SHT_ERR_UNSUPPORTED, "contracted block grid too large");
+    kspan *= nb;
+  }
+  ka.nf = (int)mp.rowA.size();
+  for (size_t t = 0; t < mp.rowA.size(); ++t) { ka.fmode[t] = mp.rowA[t]; ka.fstride[t] = C->gstride[mp.rowC[t]]; }
+  kb.nf = (int)mp.colB.size();
+  for (size_t t = 0; t < mp.colB.size(); ++t) { kb.fmode[t] = mp.colB[t]; kb.fstride[t] = C->gstride[mp.colC[t]]; }
+  cgrid = 1;
+  for (int d = 0; d < C->order; ++d) cgrid *= C->nblk[d];
+  if (cgrid > 9.0e18L) fail(SHT_ERR_UNSUPPORTED, "C block grid too large");
+}
+
+// Launches k_match on s when the grids are small enough (and the pool has room for its workspace);
+// plan_build finishes the plan from it.  Called early by callers that have other work to queue.
+void plan_match_begin(sht_plan* p, cudaStream_t s) {
+  sht_tensor *A = p->A, *B = p->B, *C = p->C;
+  const long long nA = A->nblocks, nB = B->nblocks, nC = C->nblocks;
+  KeySpec ka, kb;
+  unsigned long long kspan;
+  long double cgrid;
+  key_specs(p, ka, kb, kspan, cgrid);
+  if (nA == 0 || nB == 0 || kspan > (unsigned long long)kMatchKeys || cgrid > (long double)kMatchCells) return;
+  if (nA > (1 << 20) || nB > (1 << 20)) return;
+  DevicePool* pool = p->ctx->pool.get();
+  for (sht_tensor* t : {A, B, C}) tensor_touch(t, s);
+  auto st = std::make_shared<MatchState>(p->ctx, s);
+  MatchArgs& g = st->g;
+  const long long nc = (long long)cgrid;
+  try {
+    size_t at = 0;
+    auto part = [&](size_t bytes) {
+      const size_t o = at;
+      at += (bytes + 15) & ~(size_t)15;
+      return o;
+    };
+    const size_t o_cks = part(nc * 8), o_eofs = part(nc * 8), o_csum = part(kMatchCtas * kMatchSums * 8),
+                 o_bucket = part(kMatchBuckets * 8), o_bcur = part(kMatchBuckets * 8), o_ccnt = part(nc * 4),
+                 o_cold = part(nc * 4), o_cidx = part(nc * 4), o_pofs = part(nc * 4), o_kcnt = part(kspan * 4),
+                 o_blist = part(nB * 4), o_keyA = part(nA * 4), o_cellA = part(nA * 4), o_kA = part(nA * 4),
+                 o_keyB = part(nB * 4), o_cellB = part(nB * 4), o_rankB = part(nB * 4);
+    st->ws = PoolBuf(pool, at, s);
+    char* w = st->ws.as<char>();
+    auto ll = [&](size_t o) { return reinterpret_cast<long long*>(w + o); };
+    auto in = [&](size_t o) { return reinterpret_cast<int*>(w + o); };
+    g.cks = ll(o_cks); g.eofs = ll(o_eofs); g.csum = ll(o_csum);
+    g.bucket = reinterpret_cast<unsigned long long*>(w + o_bucket);
+    g.bcur = reinterpret_cast<unsigned long long*>(w + o_bcur);
+    g.ccnt = in(o_ccnt); g.cold = in(o_cold); g.cidx = in(o_cidx); g.pofs = in(o_pofs); g.kcnt = in(o_kcnt);
+    g.blist = in(o_blist); g.keyA = in(o_keyA); g.cellA = in(o_cellA); g.kA = in(o_kA);
+    g.keyB = in(o_keyB); g.cellB = in(o_cellB); g.rankB = in(o_rankB);
+    if (p->eps > 0.0) {
+      st->normA = PoolBuf(pool, nA * 8, s);
+      st->normB = PoolBuf(pool, nB * 8, s);
+      tensor_norms_device(A, p->norm, st->normA.as<double>(), s);
+      tensor_norms_device(B, p->norm, st->normB.as<double>(), s);
+      g.normA = st->normA.as<double>();
+      g.normB = st->normB.as<double>();
+    }
+  } catch (const Error& e) {
+    st->done = true;
+    if (e.code == SHT_ERR_OOM) return;  // the general path needs less at a time, and reports it
+    throw;
+  }
+  g.mA = make_meta(A); g.mB = make_meta(B); g.mC = make_meta(C);
+  g.ka = ka; g.kb = kb;
+  g.row = make_modemap(p->maps.rowA, p->maps.rowC);
+  g.col = make_modemap(p->maps.colB, p->maps.colC);
+  g.idsA = A->d_ids.as<long long>(); g.idsB = B->d_ids.as<long long>(); g.idsC = C->d_ids.as<long long>();
+  g.nA = nA; g.nB = nB; g.nC = nC;
+  g.eps = p->eps;
+  g.ncell = (int)nc;
+  g.kspan = (int)kspan;
+  g.tiles = p->mode != SHT_MODE_SPLIT;
+  if (p->mode == SHT_MODE_BATCHED_FP64 && !p->ctx->tuned.empty()) st->table = tuned_table(p->ctx, s);
+  g.table = st->table.as<unsigned char>();
+  void* dev = nullptr;
+  SHT_CUDA(cudaHostGetDevicePointer(&dev, st->pin.host, 0));
+  g.out = static_cast<long long*>(dev);
+  k_match<<<kMatchCtas, kMatchThreads, 0, s>>>(g);
+  const cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) {
+    st->done = true;
+    fail(SHT_ERR_CUDA, std::string("k_match: ") + cudaGetErrorString(e));
+  }
+  p->match = std::move(st);
+}
+
+// The plan from k_match's totals: allocations, C's grown pattern, pairs, work list.  False when the
+// pool has no room (nothing is changed then).
+static bool match_finish(sht_plan* p, cudaStream_t s) {
+  const std::shared_ptr<MatchState> st = std::move(p->match);
+  p->match.reset();
+  DevicePool* pool = p->ctx->pool.get();
+  sht_tensor *A = p->A, *B = p->B, *C = p->C;
+  SHT_CUDA(cudaStreamSynchronize(s));
+  st->done = true;
+  long long tot[kMatchSums];
+  for (int i = 0; i < kMatchSums; ++i) tot[i] = static_cast<volatile long long*>(st->pin.host)[i];
+  const long long np = tot[0], nc = tot[1], nwork = tot[3] + tot[4], nC_old = C->nblocks;
+  const bool grow = tot[6] > 0, fp64 = p->mode != SHT_MODE_SPLIT;
+  if (np > (long long)INT32_MAX) fail(SHT_ERR_UNSUPPORTED, "more than 2^31 block pairs");
+  if (nwork > (long long)INT32_MAX) fail(SHT_ERR_UNSUPPORTED, "work list above 2^31 tiles");
+  PoolBuf pa, pb, recs, pstart, cm, cn, ck, tmp, work, counter, ids, offs, dims, data;
+  try {
+    if (np > 0) {
+      pa = PoolBuf(pool, np * 4, s);
+      pb = PoolBuf(pool, np * 4, s);
+      if (fp64) recs = PoolBuf(pool, np * sizeof(PairRec), s);
+      tmp = PoolBuf(pool, np * 12, s);
+    }
+    pstart = PoolBuf(pool, (nc + 1) * 4, s);
+    cm = PoolBuf(pool, std::max(nc, 1LL) * 4, s);
+    cn = PoolBuf(pool, std::max(nc, 1LL) * 4, s);
+    ck = PoolBuf(pool, std::max(nc, 1LL) * 8, s);
+    if (fp64) {
+      work = PoolBuf(pool, std::max(nwork, 1LL) * sizeof(int4), s);
+      counter = PoolBuf(pool, 256, s);
+    }
+    if (grow) {
+      ids = PoolBuf(pool, nc * 8, s);
+      offs = PoolBuf(pool, nc * 8, s);
+      dims = PoolBuf(pool, nc * C->order * 4, s);
+      data = PoolBuf(pool, std::max(tot[2], 1LL) * 8, s);
+    }
+  } catch (const Error& e) {
+    if (e.code == SHT_ERR_OOM) return false;
+    throw;
+  }
+  MatchOut o{};
+  o.pstart = pstart.as<int>();
+  o.cm = cm.as<int>();
+  o.cn = cn.as<int>();
+  o.cksum = ck.as<long long>();
+  o.tmp_a = tmp.as<int>();
+  o.tmp_b = o.tmp_a + np;
+  o.tmp_c = o.tmp_b + np;
+  o.ids = ids.as<long long>();
+  o.offs = offs.as<long long>();
+  o.dims = dims.as<int>();
+  o.work = work.as<int4>();
+  o.counter = counter.as<unsigned>();
+  o.npairs = np;
+  o.nblocks = nc;
+  const long long warps = std::max<long long>((st->g.ncell + 31) / 32, st->g.nA);
+  k_match_cells<<<(unsigned)std::min<long long>((warps + 7) / 8, p->ctx->num_sms * 2LL), 256, 0, s>>>(st->g, o);
+  if (np > 0)
+    k_match_pairs<<<grid_for(np, 256), 256, 0, s>>>(
+        o, rec_modes(A->order, p->maps.rowA, p->maps.colA), rec_modes(B->order, p->maps.colB, p->maps.rowB),
+        A->d_offsets.as<long long>(), A->d_dims.as<int>(), B->d_offsets.as<long long>(), B->d_dims.as<int>(),
+        pa.as<int>(), pb.as<int>(), recs.as<PairRec>());
+  SHT_CUDA(cudaGetLastError());
+  if (grow) {
+    // C's old blocks may still be in use by earlier work on the caller's stream
+    if (nC_old > 0 && p->caller_event) SHT_CUDA(cudaStreamWaitEvent(s, p->caller_event, 0));
+    // new blocks start zero-filled, unless the caller writes every element next with nothing left
+    // that could fail for want of memory (the FP64 forms: their work list and counter are here)
+    if (!(p->c_overwritten && fp64)) {
+      SHT_CUDA(cudaMemsetAsync(data.ptr, 0, std::max(tot[2], 1LL) * 8, s));
+      if (nC_old > 0) {
+        const int grid = (int)std::min<long long>(nC_old, (long long)p->ctx->num_sms * 8);
+        k_move_blocks<double><<<grid, 256, 0, s>>>(C->d_data.as<double>(), C->d_ids.as<long long>(),
+                                                   C->d_offsets.as<long long>(), C->d_dims.as<int>(), C->order, nC_old,
+                                                   ids.as<long long>(), nc, offs.as<long long>(), data.as<double>());
+        SHT_CUDA(cudaGetLastError());
+      }
+    }
+    C->d_ids = std::move(ids);
+    C->d_offsets = std::move(offs);
+    C->d_dims = std::move(dims);
+    C->d_data = std::move(data);
+    C->nblocks = nc;
+    C->nnz = tot[2];
+    // the host mirror is read back when a host-side step needs it (no block of it is marked)
+    C->host_stale = C->stale_unmarked = true;
+    p->index_pending = true;
+  }
+  p->d_pair_a = std::move(pa);
+  p->d_pair_b = std::move(pb);
+  p->d_recs = std::move(recs);
+  p->d_pstart = std::move(pstart);
+  p->d_cm = std::move(cm);
+  p->d_cn = std::move(cn);
+  p->d_cksum = std::move(ck);
+  p->npairs = np;
+  p->ncblk = nc;
+  p->flops = (double)tot[5];
+  p->flops_pending = false;
+  if (fp64) {
+    p->d_bwork = std::move(work);
+    p->d_counter = std::move(counter);
+    p->bwork = nwork;
+    p->bwork_touched = tot[3];
+    p->work_ready = true;
+  }
+  return true;
+}
+
+void plan_settle(sht_plan* p, cudaStream_t s) {
+  if (!p->index_pending) return;
+  SHT_CUDA(cudaStreamSynchronize(s));
+  p->index_pending = false;
+}
+
 sht_plan* plan_create(sht_ctx* ctx, const std::string& expr, sht_tensor* A, sht_tensor* B, sht_tensor* C,
                       double eps, sht_norm norm, sht_mode mode, cudaStream_t s) {
   std::unique_ptr<sht_plan> p(plan_init(ctx, expr, A, B, C, eps, norm, mode, s));
   plan_build(p.get(), s);
+  plan_settle(p.get(), s);
   return p.release();
 }
 
@@ -373,7 +981,8 @@ sht_plan* plan_init(sht_ctx* ctx, const std::string& expr, sht_tensor* A, sht_te
   if (A == C || B == C) fail(SHT_ERR_INVALID, "C must not alias A or B");
   for (sht_tensor* t : {A, B, C}) {
     tensor_touch(t, s);
-    tensor_sync_host(t, s);
+    // a pattern grown by a contraction is known to be unmarked: C's host mirror can stay behind
+    if (t != C || !t->stale_unmarked) tensor_sync_host(t, s);
     if (t->has_marked) fail(SHT_ERR_STATE, "tensor has filtered blocks that were not compressed");
   }
   auto p = std::make_unique<sht_plan>();
@@ -404,25 +1013,24 @@ void plan_build(sht_plan* p, cudaStream_t s, bool speculate) {
   DevicePool* pool = ctx->pool.get();
   const long long nA = A->nblocks, nB = B->nblocks;
 
-  // contracted key radices
-  KeySpec ka{}, kb{};
-  unsigned long long kspan = 1;
-  ka.nk = kb.nk = (int)mp.colA.size();
-  for (size_t t = 0; t < mp.colA.size(); ++t) {
-    ka.kmode[t] = mp.colA[t];
-    kb.kmode[t] = mp.rowB[t];
-    ka.kstride[t] = kb.kstride[t] = (long long)kspan;
-    const unsigned long long nb = (unsigned long long)A->nblk[mp.colA[t]];
-    if (kspan > (1ULL << 62) / nb) fail(SHT_ERR_UNSUPPORTED, "contracted block grid too large");
-    kspan *= nb;
+  p->tmaps.row = make_modemap(mp.rowA, mp.rowC);
+  p->tmaps.kk = make_modemap(mp.colA, mp.rowB);
+  p->tmaps.col = make_modemap(mp.colB, mp.colC);
+  p->tmaps.oA = A->order;
+  p->tmaps.oB = B->order;
+  p->tmaps.oC = C->order;
+  if (!p->match) plan_match_begin(p, s);
+  if (p->match && match_finish(p, s)) {
+    trace("plan: matched", s);
+    p->plan_ms += now_ms() - t0;
+    return;
   }
-  ka.nf = (int)mp.rowA.size();
-  for (size_t t = 0; t < mp.rowA.size(); ++t) { ka.fmode[t] = mp.rowA[t]; ka.fstride[t] = C->gstride[mp.rowC[t]]; }
-  kb.nf = (int)mp.colB.size();
-  for (size_t t = 0; t < mp.colB.size(); ++t) { kb.fmode[t] = mp.colB[t]; kb.fstride[t] = C->gstride[mp.colC[t]]; }
-  long double cgrid = 1;
-  for (int d = 0; d < C->order; ++d) cgrid *= C->nblk[d];
-  if (cgrid > 9.0e18L) fail(SHT_ERR_UNSUPPORTED, "C block grid too large");
+
+  // contracted key radices
+  KeySpec ka, kb;
+  unsigned long long kspan;
+  long double cgrid;
+  key_specs(p, ka, kb, kspan, cgrid);
 
   // Without screening the pair count follows from the host patterns (per contracted key the
   // number of B blocks, summed over A's blocks), so the device count need not be read back.
@@ -629,13 +1237,6 @@ void plan_build(sht_plan* p, cudaStream_t s, bool speculate) {
   k_pstart<<<grid_for(nc + 1, 256), 256, 0, s>>>(C->d_ids.as<long long>(), nc, pc_sorted.as<long long>(), np,
                                                   p->d_pstart.as<int>());
   SHT_CUDA(cudaGetLastError());
-  p->flops = 0;
-  p->tmaps.row = make_modemap(mp.rowA, mp.rowC);
-  p->tmaps.kk = make_modemap(mp.colA, mp.rowB);
-  p->tmaps.col = make_modemap(mp.colB, mp.colC);
-  p->tmaps.oA = A->order;
-  p->tmaps.oB = B->order;
-  p->tmaps.oC = C->order;
   // per C block m, n, sum of the pairs' k and flops; the total flop count
   cblock_stats(p, s);
   trace("plan: pstart+flops", s);

@@ -4,6 +4,10 @@
 #include "sht_internal.h"
 #include "tile_types.h"
 
+namespace sht {
+struct MatchState;
+}
+
 struct sht_plan {
   std::shared_ptr<sht::DevicePool> keep;  // declared first: released after the buffers below
   sht_ctx* ctx = nullptr;
@@ -44,11 +48,14 @@ struct sht_plan {
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t graph_exec = nullptr;
   double graph_alpha = 0.0, graph_beta = 0.0;
-  ~sht_plan() {
-    if (graph_exec) cudaGraphExecDestroy(graph_exec);
-    if (graph) cudaGraphDestroy(graph);
-    if (flops_event) cudaEventDestroy(flops_event);
-  }
+  // plans over small block grids (contract.cu): the counting kernel in flight, what it left to do
+  std::shared_ptr<sht::MatchState> match;
+  bool work_ready = false;     // the work list came with the pairs
+  bool c_overwritten = false;  // the caller writes every element of C next: no zero fill, no move
+  cudaEvent_t caller_event = nullptr;  // earlier work on the caller's stream, when the build has its own
+  bool index_pending = false;  // C's new index is still being written (plan_settle)
+  sht_plan();
+  ~sht_plan();
 };
 
 namespace sht {
@@ -64,6 +71,12 @@ sht_plan* plan_init(sht_ctx* ctx, const std::string& expr, sht_tensor* A, sht_te
 // saves a synchronization when C is contracted into repeatedly.
 void plan_build(sht_plan* p, cudaStream_t s, bool speculate = false);
 struct PatternGrew {};
+// starts the plan's counting kernel on s ahead of plan_build (small block grids; else nothing)
+void plan_match_begin(sht_plan* p, cudaStream_t s);
+// waits for a grown C index to be written: calls return with every index complete
+void plan_settle(sht_plan* p, cudaStream_t s);
+// the autotuner's choices as a device table (class_index)
+PoolBuf tuned_table(sht_ctx* ctx, cudaStream_t s);
 void cblock_stats(sht_plan* p, cudaStream_t s);
 // The plan's flop count; the first call after planning copies it from the device (a sync),
 // so callers that synchronize anyway read it right after.

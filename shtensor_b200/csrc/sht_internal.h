@@ -171,6 +171,8 @@ struct sht_ctx {
   };
   std::mutex lanes_mu;
   std::vector<Lane> lanes;
+  std::vector<long long*> pins;         // free slots of host-mapped memory (128 bytes; lanes_mu)
+  std::vector<void*> pin_pages;
   std::map<std::string, int> tuned;     // autotuner choices: size-class key -> tile id
   int split_slices = 0;                 // INT8 slices per operand in split mode (0 = default)
   long long wait_limit = 0;             // polls of a device pipeline wait (0 = default)
@@ -210,6 +212,7 @@ struct sht_tensor {
   // host index (authoritative unless host_stale)
   std::vector<int64_t> ids, offsets, rows;
   bool host_stale = false;
+  bool stale_unmarked = false;  // host_stale, and known to hold no filtered id
   bool has_marked = false;  // the host index holds filtered (negative) ids
   // per-block extents and block-grid coordinates (nblocks x order each) of the host index,
   // computed on first use after the host index changes (tensor_host_dims, tensor_host_coords)

@@ -82,7 +82,7 @@ void tensor_set_index(sht_tensor* t, std::vector<int64_t>&& ids, cudaStream_t s)
     int64_t acc = 0;
     for (int r = 0; r < t->nblk[0]; ++r) { t->rows[r] = acc; acc += cnt[r]; }
   }
-  t->host_stale = false;
+  t->host_stale = t->stale_unmarked = false;
   t->d_ids = PoolBuf(pool, std::max<int64_t>(t->nblocks, 1) * 8, s);
   t->d_offsets = PoolBuf(pool, std::max<int64_t>(t->nblocks, 1) * 8, s);
   t->d_dims = PoolBuf(pool, std::max<int64_t>(t->nblocks, 1) * t->order * 4, s);
@@ -243,6 +243,7 @@ void tensor_sync_host(sht_tensor* t, cudaStream_t s) {
     cnt[(id >= 0 ? id : -(id + 1)) % t->nblk[0]]++;  // marked ids are -(id)-1
   }
   t->has_marked = marked;
+  t->stale_unmarked = false;
   int64_t acc = 0;
   for (int r = 0; r < t->nblk[0]; ++r) { t->rows[r] = acc; acc += cnt[r]; }
   t->host_stale = false;

@@ -34,6 +34,37 @@ __host__ __device__ constexpr int ring_tn(int s) { return s & 1 ? 32 : 64; }
 __host__ __device__ __forceinline__ int ring_ntiles(int ext, int t) { return (ext + t - 1) / t; }
 __host__ __device__ __forceinline__ int ring_step(int ext, int nt) { return (((ext + nt - 1) / nt) + 7) & ~7; }
 
+// Cost of one C block per unit of contracted extent in a tile shape, in products: what the tensor
+// pipe runs (the tile's fragments of 8x8, and four times the busiest warp's, averaged: a tile
+// waits for its busiest warp, but another CTA fills the gap), the operand copies, and a fixed
+// cost per tile.
+__host__ __device__ inline float shape_cost(int m, int n, int sh) {
+  const int ntr = ring_ntiles(m, ring_tm(sh)), ntc = ring_ntiles(n, ring_tn(sh));
+  const int fr = ring_step(m, ntr) / 8, fc = ring_step(n, ntc) / 8;
+  const float busiest = 4.0f * (float)(((fr + 1) / 2) * ((fc + 1) / 2));
+  return (float)ntr * (float)ntc * (32.0f * ((float)(fr * fc) + busiest) + 64.0f * (float)(fr + fc) + 512.0f);
+}
+__host__ __device__ inline int model_shape(int m, int n) {
+  float best = 3.0e38f;
+  int bi = 0;
+  for (int s = 0; s < kRingShapes; ++s) {
+    const float c = shape_cost(m, n, s);
+    if (c < best) { best = c; bi = s; }
+  }
+  return bi;
+}
+
+// Size class of a C block in the autotuner's table: ceil(log2) of its rows, columns and mean contracted
+// extent, 32 values each.
+__host__ __device__ inline int ilog2_up(long long v) {
+  int b = 0;
+  while (b < 31 && (1LL << b) < v) ++b;
+  return b;
+}
+__host__ __device__ inline int class_index(int m, int n, long long kavg) {
+  return (ilog2_up(m) * 32 + ilog2_up(n)) * 32 + ilog2_up(kavg > 0 ? kavg : 1);
+}
+
 // One block pair of a plan as the FP64 kernel reads it: where its blocks start, the contracted extent
 // and the strides of linear addressing (tile_ring.cuh).  Built once per pair; every tile of the pair's
 // C block reads it.
