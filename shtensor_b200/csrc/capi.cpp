@@ -57,6 +57,8 @@ static void contract_split(sht_plan* p, double alpha, double beta, cudaStream_t 
   // without screening the counting kernel of the plan goes ahead of the slicer, whose CTAs fill the SMs
   if (!(p->eps > 0.0)) plan_match_begin(p, ps);
   split_layout(p, ctx->split_slices ? ctx->split_slices : split_slices_default(), s);
+  // the records below read the layout's upload, which waits on s for the work queued there
+  SHT_CUDA(cudaEventRecord(lane.lane.done, s));
   split_slice(p, alpha, s);
   trace("contract: slicer launched", s);
   // The build reads the tensors' indices (complete: every index change in this library returns
@@ -66,6 +68,7 @@ static void contract_split(sht_plan* p, double alpha, double beta, cudaStream_t 
   if (p->eps > 0.0) SHT_CUDA(cudaStreamWaitEvent(ps, lane.lane.start, 0));
   try {
     plan_build(p, ps, true);
+    SHT_CUDA(cudaStreamWaitEvent(ps, lane.lane.done, 0));
     split_records(p, ps);
   } catch (const PatternGrew&) {
     // the product adds blocks to C: build again, growing C's pattern, which moves C's values

@@ -281,8 +281,10 @@ __global__ void k_count_missing(const long long* __restrict__ pc, long long np, 
 constexpr int kMatchCtas = 8, kMatchThreads = 1024;
 constexpr long long kMatchCells = 1 << 18;  // C's block grid
 constexpr int kMatchKeys = 512;             // contracted block grid: also the most pairs of one cell
-constexpr int kMatchBuckets = 65;           // cost classes of work items, heaviest first; last: untouched
-constexpr int kMatchSums = 7;               // pairs, blocks, elements, tiles touched / untouched, flops, new blocks
+constexpr int kMatchBuckets = 1024;         // classes of work items in list order; last: untouched blocks
+constexpr int kMatchCosts = 64;             // cost classes, heaviest first
+constexpr int kMatchSums = 9;               // pairs, blocks, elements, tiles touched / untouched, flops, new blocks,
+                                            // row and column table entries (split plans)
 
 struct MatchArgs {
   TensorMeta mA, mB, mC;
@@ -295,11 +297,13 @@ struct MatchArgs {
   const double *normA, *normB;  // null: no screening
   double eps;
   int ncell, kspan;
-  int tiles;                     // count tiles and order them (FP64 forms)
+  int split_m, split_n;          // split plans: the tile (128 x 32); 0: the FP64 forms' shapes
+  int many;                      // split plans: this many blocks are listed by row coordinates, fewer by cost
+  int row_span;                  // positions of the row modes' block grid
   const unsigned char* table;    // the autotuner's shapes (null: the model's)
   // workspace
   int *kcnt, *blist, *keyA, *cellA, *kA, *keyB, *cellB, *rankB;
-  int *ccnt, *cold, *cidx, *pofs;
+  int *ccnt, *cold, *cidx, *pofs, *rofs, *cofs, *nocc;
   long long *cks, *eofs, *csum;
   unsigned long long *bucket, *bcur;
   long long* out;                // kMatchSums totals, host-mapped
@@ -315,27 +319,44 @@ struct MatchCell {
   int m, n, sh, nt, bucket;
   long long elems;
 };
-__device__ __forceinline__ MatchCell match_cell(const MatchArgs& g, int cell, int np, long long ks) {
+__device__ __forceinline__ MatchCell match_cell(const MatchArgs& g, int cell, int np, long long ks, bool by_row) {
   MatchCell c{1, 1, 0, 0, 0, 1};
+  int row = 0, mul = 1;
   for (int t = 0; t < g.row.n; ++t) {
-    const int y = g.row.y[t];
-    c.m *= g.mC.bsizes[g.mC.bstart[y] + cell / (int)g.mC.gstride[y] % g.mC.nblk[y]];
+    const int y = g.row.y[t], x = cell / (int)g.mC.gstride[y] % g.mC.nblk[y];
+    c.m *= g.mC.bsizes[g.mC.bstart[y] + x];
+    row += x * mul;
+    mul *= g.mC.nblk[y];
   }
   for (int t = 0; t < g.col.n; ++t) {
     const int y = g.col.y[t];
     c.n *= g.mC.bsizes[g.mC.bstart[y] + cell / (int)g.mC.gstride[y] % g.mC.nblk[y]];
   }
   c.elems = (long long)c.m * c.n;
-  if (g.tiles) {
+  int ntr, ntc, sr, sc;
+  if (g.split_m) {
+    ntr = (c.m + g.split_m - 1) / g.split_m;
+    ntc = (c.n + g.split_n - 1) / g.split_n;
+    sr = g.split_m;
+    sc = g.split_n;
+  } else {
     int t = 255;
     if (g.table) t = g.table[class_index(c.m, c.n, np > 0 ? ks / np : 1)];
     c.sh = t != 255 ? t : model_shape(c.m, c.n);
-    const int ntr = ring_ntiles(c.m, ring_tm(c.sh)), ntc = ring_ntiles(c.n, ring_tn(c.sh));
-    c.nt = ntr * ntc;
-    // cost of a tile in half octaves, heaviest first
-    const float cost = (float)ring_step(c.m, ntr) * (float)ring_step(c.n, ntc) * (float)ks + 1.0f;
-    c.bucket = np > 0 ? kMatchBuckets - 2 - min(kMatchBuckets - 2, (int)(__float_as_uint(cost) >> 22) - 254)
-                      : kMatchBuckets - 1;
+    ntr = ring_ntiles(c.m, ring_tm(c.sh));
+    ntc = ring_ntiles(c.n, ring_tn(c.sh));
+    sr = ring_step(c.m, ntr);
+    sc = ring_step(c.n, ntc);
+  }
+  c.nt = ntr * ntc;
+  if (np == 0) {
+    c.bucket = kMatchBuckets - 1;
+  } else if (by_row) {  // blocks that read the same A slabs run close together in time
+    const int span = min(g.row_span, kMatchBuckets - 1);
+    c.bucket = (int)((long long)row * span / g.row_span);
+  } else {  // cost of a tile in half octaves, heaviest first
+    const float cost = (float)sr * (float)sc * (float)ks + 1.0f;
+    c.bucket = kMatchCosts - 1 - min(kMatchCosts - 1, (int)(__float_as_uint(cost) >> 22) - 254);
   }
   return c;
 }
@@ -363,16 +384,21 @@ __device__ __forceinline__ T match_scan(T v, T* scratch) {
   return warp ? v + scratch[warp - 1] : v;
 }
 
-// the surviving pairs of A block a, a warp at a time: f(b, cell)
+// the surviving pairs of A block a, `width` lanes at a time (lane: this thread's among them): f(b, cell)
 template <class F>
-__device__ __forceinline__ void match_pairs_of(const MatchArgs& g, const int* kstart, int a, int lane, F f) {
+__device__ __forceinline__ void match_pairs_of(const MatchArgs& g, const int* kstart, int a, int lane, int width, F f) {
   const int k = g.keyA[a], cell = g.cellA[a];
   const double na = g.normA ? g.normA[a] : 0.0;
-  for (int j = kstart[k] + lane; j < kstart[k + 1]; j += 32) {
+  for (int j = kstart[k] + lane; j < kstart[k + 1]; j += width) {
     const int b = g.blist[j];
     if (g.normA && !(na * g.normB[b] >= g.eps)) continue;
     f(b, cell + g.cellB[b]);
   }
+}
+// lanes per A block: about the mean length of a key's B list
+__device__ __forceinline__ int match_width(const MatchArgs& g) {
+  const long long mean = g.nB / g.kspan;
+  return mean <= 4 ? 4 : mean <= 8 ? 8 : mean <= 16 ? 16 : 32;
 }
 
 __device__ __forceinline__ void match_kstart(const MatchArgs& g, int* kstart) {
@@ -409,7 +435,8 @@ __global__ void __cluster_dims__(kMatchCtas, 1, 1) __launch_bounds__(kMatchThrea
     g.cks[i] = 0;
   }
   if (gt < kMatchBuckets) g.bucket[gt] = g.bcur[gt] = 0;
-  if (threadIdx.x < kMatchBuckets) hist[threadIdx.x] = 0;
+  if (gt == 0) *g.nocc = 0;
+  hist[threadIdx.x] = 0;
   if (threadIdx.x < kMatchSums) sums[threadIdx.x] = 0;
   match_sync();
   // keys and C parts of the operands' blocks; C's stored cells
@@ -444,28 +471,40 @@ __global__ void __cluster_dims__(kMatchCtas, 1, 1) __launch_bounds__(kMatchThrea
   for (int b = gt; b < g.nB; b += nt) g.blist[kstart[g.keyB[b]] + g.rankB[b]] = b;
   match_sync();
   // pairs per cell and their contracted extents
-  for (int a = gt >> 5; a < g.nA; a += nt >> 5)
-    match_pairs_of(g, kstart, a, lane, [&](int, int cell) {
+  const int width = match_width(g);
+  for (int a = gt / width; a < g.nA; a += nt / width)
+    match_pairs_of(g, kstart, a, lane & (width - 1), width, [&](int, int cell) {
       atomicAdd(&g.ccnt[cell], 1);
       atomicAdd(reinterpret_cast<unsigned long long*>(&g.cks[cell]), (unsigned long long)g.kA[a]);
     });
   match_sync();
-  // totals of this CTA's range of cells, and the cost classes
   const int per = (g.ncell + kMatchCtas - 1) / kMatchCtas, c0 = min(g.ncell, cta * per), c1 = min(g.ncell, c0 + per);
+  bool by_row = false;
+  if (g.split_m) {
+    int occ = 0;
+    for (int cell = c0 + threadIdx.x; cell < c1; cell += kMatchThreads) occ += g.ccnt[cell] || g.cold[cell];
+    for (int d = 16; d; d >>= 1) occ += __shfl_xor_sync(0xffffffffu, occ, d);
+    if (lane == 0 && occ) atomicAdd(g.nocc, occ);
+    match_sync();
+    by_row = *static_cast<volatile int*>(g.nocc) >= g.many;
+  }
+  // totals of this CTA's range of cells, and the classes
   {
-    long long v[kMatchSums] = {0, 0, 0, 0, 0, 0, 0};
+    long long v[kMatchSums] = {};
     for (int cell = c0 + threadIdx.x; cell < c1; cell += kMatchThreads) {
       const int np = g.ccnt[cell], old = g.cold[cell];
       if (!np && !old) continue;
       const long long ks = g.cks[cell];
-      const MatchCell c = match_cell(g, cell, np, ks);
+      const MatchCell c = match_cell(g, cell, np, ks, by_row);
       v[0] += np;
       v[1] += 1;
       v[2] += c.elems;
       v[np ? 3 : 4] += c.nt;
       v[5] += 2 * c.elems * ks;
       v[6] += old ? 0 : 1;
-      if (g.tiles) atomicAdd(&hist[c.bucket], (unsigned long long)c.nt);
+      v[7] += (c.m + 3) & ~3;
+      v[8] += (c.n + 3) & ~3;
+      atomicAdd(&hist[c.bucket], (unsigned long long)c.nt);
     }
 #pragma unroll
     for (int i = 0; i < kMatchSums; ++i) {
@@ -474,41 +513,65 @@ __global__ void __cluster_dims__(kMatchCtas, 1, 1) __launch_bounds__(kMatchThrea
     }
     __syncthreads();
     if (threadIdx.x < kMatchSums) g.csum[cta * kMatchSums + threadIdx.x] = sums[threadIdx.x];
-    if (threadIdx.x < kMatchBuckets && hist[threadIdx.x]) atomicAdd(&g.bucket[threadIdx.x], hist[threadIdx.x]);
+    if (hist[threadIdx.x]) atomicAdd(&g.bucket[threadIdx.x], hist[threadIdx.x]);
   }
   match_sync();
-  // positions: pairs before each cell, its block number, its first element
-  long long base[3] = {0, 0, 0};
-  for (int r = 0; r < cta; ++r)
-    for (int i = 0; i < 3; ++i) base[i] += g.csum[r * kMatchSums + i];
+  // positions: pairs before each cell, its block number, its first element, its first table entries
+  __shared__ long long base[5];
+  if (threadIdx.x < 5) {
+    const int i = threadIdx.x < 3 ? threadIdx.x : threadIdx.x + 4;
+    long long v = 0;
+    for (int r = 0; r < cta; ++r) v += g.csum[r * kMatchSums + i];
+    base[threadIdx.x] = v;
+  }
+  __syncthreads();
   for (int lo = c0; lo < c1; lo += kMatchThreads) {
     const int cell = lo + threadIdx.x;
-    int np = 0, occ = 0;
+    int np = 0, occ = 0, rm = 0, rn = 0;
     long long el = 0;
     if (cell < c1) {
       np = g.ccnt[cell];
       occ = np || g.cold[cell] ? 1 : 0;
       if (occ) {
-        el = 1;
-        for (int d = 0; d < g.mC.order; ++d)
-          el *= g.mC.bsizes[g.mC.bstart[d] + cell / (int)g.mC.gstride[d] % g.mC.nblk[d]];
+        int m = 1, n = 1;
+        for (int t = 0; t < g.row.n; ++t) {
+          const int y = g.row.y[t];
+          m *= g.mC.bsizes[g.mC.bstart[y] + cell / (int)g.mC.gstride[y] % g.mC.nblk[y]];
+        }
+        for (int t = 0; t < g.col.n; ++t) {
+          const int y = g.col.y[t];
+          n *= g.mC.bsizes[g.mC.bstart[y] + cell / (int)g.mC.gstride[y] % g.mC.nblk[y]];
+        }
+        el = (long long)m * n;
+        rm = (m + 3) & ~3;
+        rn = (n + 3) & ~3;
       }
     }
     const int pi = match_scan(np, iscratch), oi = match_scan(occ, iscratch);
     const long long ei = match_scan(el, scratch);
+    int ri = 0, ni = 0;
+    if (g.split_m) {
+      ri = match_scan(rm, iscratch);
+      ni = match_scan(rn, iscratch);
+    }
     if (cell < c1) {
       g.pofs[cell] = (int)base[0] + pi - np;
       g.cidx[cell] = occ ? (int)base[1] + oi - 1 : -1;
       g.eofs[cell] = base[2] + ei - el;
+      if (g.split_m) {
+        g.rofs[cell] = (int)(base[3] + ri - rm);
+        g.cofs[cell] = (int)(base[4] + ni - rn);
+      }
     }
     __syncthreads();
     if (threadIdx.x == kMatchThreads - 1) {
-      sums[0] = pi;
-      sums[1] = oi;
-      sums[2] = ei;
+      base[0] += pi;
+      base[1] += oi;
+      base[2] += ei;
+      base[3] += ri;
+      base[4] += ni;
     }
     __syncthreads();
-    for (int i = 0; i < 3; ++i) base[i] += sums[i];
   }
   if (cta == 0 && threadIdx.x < kMatchSums) {
     long long v = 0;
@@ -524,25 +587,40 @@ struct MatchOut {
   long long* cksum;
   long long *ids, *offs;  // C's new index (null: the pattern is unchanged)
   int* dims;
-  int4* work;             // null: no work list
-  unsigned* counter;
+  int4* work;
+  unsigned* counter;      // the FP64 forms' (null in split plans)
+  long long *rowbase, *colbase;  // split plans: first entry of each block in the row / column tables
   long long npairs, nblocks;
 };
 __global__ void __launch_bounds__(256) k_match_cells(const __grid_constant__ MatchArgs g, MatchOut o) {
   __shared__ int kstart[kMatchKeys + 1];
   __shared__ unsigned long long bstart[kMatchBuckets];
   match_kstart(g, kstart);
-  if (threadIdx.x == 0) {
-    unsigned long long s = 0;
-    for (int i = 0; i < kMatchBuckets; ++i) {
-      bstart[i] = s;
-      s += g.bucket[i];
+  {  // starts of the classes: four per thread
+    __shared__ unsigned long long wsum[8];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    unsigned long long v[4], t = 0;
+    for (int i = 0; i < 4; ++i) {
+      v[i] = t;
+      t += g.bucket[4 * threadIdx.x + i];
     }
-    if (blockIdx.x == 0) {
-      o.pstart[o.nblocks] = (int)o.npairs;
-      if (o.counter) *o.counter = 0;
+    unsigned long long x = t;
+    for (int d = 1; d < 32; d <<= 1) {
+      const unsigned long long y = __shfl_up_sync(0xffffffffu, x, d);
+      if (lane >= d) x += y;
     }
+    if (lane == 31) wsum[warp] = x;
+    __syncthreads();
+    unsigned long long before = x - t;
+    for (int w = 0; w < warp; ++w) before += wsum[w];
+    for (int i = 0; i < 4; ++i) bstart[4 * threadIdx.x + i] = before + v[i];
   }
+  static_assert(kMatchBuckets == 4 * 256, "four classes per thread");
+  if (threadIdx.x == 0 && blockIdx.x == 0) {
+    o.pstart[o.nblocks] = (int)o.npairs;
+    if (o.counter) *o.counter = 0;
+  }
+  const bool by_row = g.split_m && *g.nocc >= g.many;
   __syncthreads();
   const int lane = threadIdx.x & 31, gw = (blockIdx.x * 256 + threadIdx.x) >> 5, nw = gridDim.x * 8;
   for (int base = gw * 32; base < g.ncell; base += nw * 32) {
@@ -553,7 +631,7 @@ __global__ void __launch_bounds__(256) k_match_cells(const __grid_constant__ Mat
     if (ci >= 0) {
       const int np = g.ccnt[cell];
       const long long ks = g.cks[cell];
-      c = match_cell(g, cell, np, ks);
+      c = match_cell(g, cell, np, ks, by_row);
       o.pstart[ci] = g.pofs[cell];
       o.cm[ci] = c.m;
       o.cn[ci] = c.n;
@@ -565,21 +643,28 @@ __global__ void __launch_bounds__(256) k_match_cells(const __grid_constant__ Mat
           o.dims[(long long)ci * g.mC.order + d] =
               g.mC.bsizes[g.mC.bstart[d] + cell / (int)g.mC.gstride[d] % g.mC.nblk[d]];
       }
-      if (o.work) w0 = bstart[c.bucket] + atomicAdd(&g.bcur[c.bucket], (unsigned long long)c.nt);
+      if (o.rowbase) {
+        o.rowbase[ci] = g.rofs[cell];
+        o.colbase[ci] = g.cofs[cell];
+      }
+      w0 = bstart[c.bucket] + atomicAdd(&g.bcur[c.bucket], (unsigned long long)c.nt);
     }
     // the cells' tiles, one cell after another, lanes over tiles
-    if (o.work)
+    {
       for (unsigned todo = __ballot_sync(0xffffffffu, ci >= 0); todo; todo &= todo - 1) {
         const int l = __ffs(todo) - 1;
         const int m = __shfl_sync(0xffffffffu, c.m, l), n = __shfl_sync(0xffffffffu, c.n, l);
         const int sh = __shfl_sync(0xffffffffu, c.sh, l), nt = __shfl_sync(0xffffffffu, c.nt, l);
         const int cc = __shfl_sync(0xffffffffu, ci, l);
         const unsigned long long w = __shfl_sync(0xffffffffu, w0, l);
-        for (int t = lane; t < nt; t += 32) o.work[w + t] = ring_item(cc, t, m, n, ring_tm(sh), ring_tn(sh));
+        for (int t = lane; t < nt; t += 32)
+          o.work[w + t] = g.split_m ? make_int4(cc, t, 0, 0) : ring_item(cc, t, m, n, ring_tm(sh), ring_tn(sh));
       }
+    }
   }
-  for (int a = gw; a < g.nA; a += nw)
-    match_pairs_of(g, kstart, a, lane, [&](int b, int cell) {
+  const int width = match_width(g);
+  for (int a = (blockIdx.x * 256 + threadIdx.x) / width; a < g.nA; a += gridDim.x * 256 / width)
+    match_pairs_of(g, kstart, a, lane & (width - 1), width, [&](int b, int cell) {
       // the old-block marks are not needed any more: the cells' cursors (from 0 or 1)
       const int slot = g.pofs[cell] + (atomicAdd(&g.cold[cell], 2) >> 1);
       o.tmp_a[slot] = a;
@@ -796,7 +881,8 @@ void plan_match_begin(sht_plan* p, cudaStream_t s) {
     };
     const size_t o_cks = part(nc * 8), o_eofs = part(nc * 8), o_csum = part(kMatchCtas * kMatchSums * 8),
                  o_bucket = part(kMatchBuckets * 8), o_bcur = part(kMatchBuckets * 8), o_ccnt = part(nc * 4),
-                 o_cold = part(nc * 4), o_cidx = part(nc * 4), o_pofs = part(nc * 4), o_kcnt = part(kspan * 4),
+                 o_cold = part(nc * 4), o_cidx = part(nc * 4), o_pofs = part(nc * 4), o_rofs = part(nc * 4),
+                 o_cofs = part(nc * 4), o_nocc = part(4), o_kcnt = part(kspan * 4),
                  o_blist = part(nB * 4), o_keyA = part(nA * 4), o_cellA = part(nA * 4), o_kA = part(nA * 4),
                  o_keyB = part(nB * 4), o_cellB = part(nB * 4), o_rankB = part(nB * 4);
     st->ws = PoolBuf(pool, at, s);
@@ -806,7 +892,7 @@ void plan_match_begin(sht_plan* p, cudaStream_t s) {
     g.cks = ll(o_cks); g.eofs = ll(o_eofs); g.csum = ll(o_csum);
     g.bucket = reinterpret_cast<unsigned long long*>(w + o_bucket);
     g.bcur = reinterpret_cast<unsigned long long*>(w + o_bcur);
-    g.ccnt = in(o_ccnt); g.cold = in(o_cold); g.cidx = in(o_cidx); g.pofs = in(o_pofs); g.kcnt = in(o_kcnt);
+    g.ccnt = in(o_ccnt); g.cold = in(o_cold); g.cidx = in(o_cidx); g.pofs = in(o_pofs); g.rofs = in(o_rofs); g.cofs = in(o_cofs); g.nocc = in(o_nocc); g.kcnt = in(o_kcnt);
     g.blist = in(o_blist); g.keyA = in(o_keyA); g.cellA = in(o_cellA); g.kA = in(o_kA);
     g.keyB = in(o_keyB); g.cellB = in(o_cellB); g.rankB = in(o_rankB);
     if (p->eps > 0.0) {
@@ -831,7 +917,12 @@ void plan_match_begin(sht_plan* p, cudaStream_t s) {
   g.eps = p->eps;
   g.ncell = (int)nc;
   g.kspan = (int)kspan;
-  g.tiles = p->mode != SHT_MODE_SPLIT;
+  if (p->mode == SHT_MODE_SPLIT) {
+    split_tile(g.split_m, g.split_n);
+    g.many = 16 * p->ctx->num_sms;
+    g.row_span = 1;
+    for (int t = 0; t < g.row.n; ++t) g.row_span *= C->nblk[g.row.y[t]];
+  }
   if (p->mode == SHT_MODE_BATCHED_FP64 && !p->ctx->tuned.empty()) st->table = tuned_table(p->ctx, s);
   g.table = st->table.as<unsigned char>();
   void* dev = nullptr;
@@ -861,7 +952,9 @@ static bool match_finish(sht_plan* p, cudaStream_t s) {
   const bool grow = tot[6] > 0, fp64 = p->mode != SHT_MODE_SPLIT;
   if (np > (long long)INT32_MAX) fail(SHT_ERR_UNSUPPORTED, "more than 2^31 block pairs");
   if (nwork > (long long)INT32_MAX) fail(SHT_ERR_UNSUPPORTED, "work list above 2^31 tiles");
-  PoolBuf pa, pb, recs, pstart, cm, cn, ck, tmp, work, counter, ids, offs, dims, data;
+  if (!fp64 && (tot[7] >= (1LL << 31) || tot[8] >= (1LL << 31)))
+    fail(SHT_ERR_UNSUPPORTED, "split mode: C row / column tables above 2^31");
+  PoolBuf pa, pb, recs, pstart, cm, cn, ck, tmp, work, counter, rowb, colb, ids, offs, dims, data;
   try {
     if (np > 0) {
       pa = PoolBuf(pool, np * 4, s);
@@ -873,9 +966,12 @@ static bool match_finish(sht_plan* p, cudaStream_t s) {
     cm = PoolBuf(pool, std::max(nc, 1LL) * 4, s);
     cn = PoolBuf(pool, std::max(nc, 1LL) * 4, s);
     ck = PoolBuf(pool, std::max(nc, 1LL) * 8, s);
+    work = PoolBuf(pool, std::max(nwork, 1LL) * sizeof(int4), s);
     if (fp64) {
-      work = PoolBuf(pool, std::max(nwork, 1LL) * sizeof(int4), s);
       counter = PoolBuf(pool, 256, s);
+    } else {
+      rowb = PoolBuf(pool, std::max(nc, 1LL) * 8, s);
+      colb = PoolBuf(pool, std::max(nc, 1LL) * 8, s);
     }
     if (grow) {
       ids = PoolBuf(pool, nc * 8, s);
@@ -900,6 +996,8 @@ static bool match_finish(sht_plan* p, cudaStream_t s) {
   o.dims = dims.as<int>();
   o.work = work.as<int4>();
   o.counter = counter.as<unsigned>();
+  o.rowbase = rowb.as<long long>();
+  o.colbase = colb.as<long long>();
   o.npairs = np;
   o.nblocks = nc;
   const long long warps = std::max<long long>((st->g.ncell + 31) / 32, st->g.nA);
@@ -946,13 +1044,15 @@ static bool match_finish(sht_plan* p, cudaStream_t s) {
   p->ncblk = nc;
   p->flops = (double)tot[5];
   p->flops_pending = false;
-  if (fp64) {
-    p->d_bwork = std::move(work);
-    p->d_counter = std::move(counter);
-    p->bwork = nwork;
-    p->bwork_touched = tot[3];
-    p->work_ready = true;
-  }
+  p->d_bwork = std::move(work);
+  p->d_counter = std::move(counter);
+  p->bwork = nwork;
+  p->bwork_touched = tot[3];
+  p->work_ready = true;
+  p->sp_rowbase = std::move(rowb);
+  p->sp_colbase = std::move(colb);
+  p->sp_rtot = tot[7];
+  p->sp_ctot = tot[8];
   return true;
 }
 
@@ -966,7 +1066,9 @@ sht_plan* plan_create(sht_ctx* ctx, const std::string& expr, sht_tensor* A, sht_
                       double eps, sht_norm norm, sht_mode mode, cudaStream_t s) {
   std::unique_ptr<sht_plan> p(plan_init(ctx, expr, A, B, C, eps, norm, mode, s));
   plan_build(p.get(), s);
-  plan_settle(p.get(), s);
+  // the pair list can be read back on another stream, and C's index by any later call
+  SHT_CUDA(cudaStreamSynchronize(s));
+  p->index_pending = false;
   return p.release();
 }
 
@@ -1263,7 +1365,7 @@ void plan_touch(sht_plan* p, cudaStream_t s) {
   for (sht_tensor* t : {p->A, p->B, p->C}) tensor_touch(t, s);
   for (PoolBuf* b : {&p->d_pair_a, &p->d_pair_b, &p->d_recs, &p->d_pstart, &p->d_bwork, &p->d_counter}) b->use_on(s);
   for (PoolBuf* b : {&p->sp_a, &p->sp_b, &p->sp_ae, &p->sp_be, &p->sp_bsc, &p->sp_meta, &p->sp_items, &p->sp_pairs,
-                     &p->sp_rowtab, &p->sp_coltab})
+                     &p->sp_rowtab, &p->sp_coltab, &p->sp_rowbase, &p->sp_colbase})
     b->use_on(s);
 }
 

@@ -42,6 +42,8 @@ struct sht_plan {
   int* sp_err = nullptr;            // the execute's flag words (non-finite input, wide exponents)
   long long sp_naitems = 0, sp_nbitems = 0;
   sht::PoolBuf sp_items, sp_pairs;    // per-tile and per-pair records of the split kernel
+  sht::PoolBuf sp_rowbase, sp_colbase;  // int64 per C block: its first entry in those tables
+  long long sp_rtot = 0, sp_ctot = 0;   // their entries
   sht::PoolBuf sp_rowtab, sp_coltab;  // element offsets of every C row / column in its block
   int split_slices = 0;
   // graph replay
@@ -125,6 +127,7 @@ void split_launch(sht_plan* p, const SparseArgs& sa, cudaStream_t s);
 void fallback_tiles_if(const SparseArgs& g, const int4* work, long long nwork, const int* flag, int grid,
                        cudaStream_t s);
 int split_slices_default();
+void split_tile(int& m, int& n);  // rows and columns of the split kernel's tiles
 // Serving: requests of one launch share the kind (slice count and reassembly instance); the
 // host buffer holds split_desc_bytes() per request; the flags are read after the slicer (a
 // synchronization of s) and must be clear for a request to join a split launch.

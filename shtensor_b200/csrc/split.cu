@@ -554,24 +554,30 @@ __global__ void k_split_offsets(const int* __restrict__ dimsC, long long nc, Til
     int m = 1, n = 1;
     for (int q = 0; q < mp.row.n; ++q) m *= cd[mp.row.y[q]];
     for (int q = 0; q < mp.col.n; ++q) n *= cd[mp.col.y[q]];
-    for (int r = lane; r < m; r += 32) {
-      int x = r, off = 0;
-      for (int q = 0; q < mp.row.n; ++q) {
-        const int e = cd[mp.row.y[q]];
-        off += (x % e) * st[mp.row.y[q]];
-        x /= e;
+    // one dimension: index x < 65536 is divided by multiplying with the rounded-up reciprocal, which
+    // is exact there (45 us of integer divisions for 18,325 blocks before)
+    auto fill = [&](const ModeMap& mm, int ext, int* out) {
+      if (mm.n <= 2 && ext < 65536) {
+        const int e = mm.n ? cd[mm.y[0]] : 1, s0 = mm.n ? st[mm.y[0]] : 0, s1 = mm.n > 1 ? st[mm.y[1]] : 0;
+        const unsigned inv = e > 1 ? 0xffffffffu / (unsigned)e + 1u : 0u;
+        for (int i = lane; i < ext; i += 32) {
+          const int q = e > 1 ? (int)__umulhi((unsigned)i, inv) : i;
+          out[i] = (i - q * e) * s0 + q * s1;
+        }
+        return;
       }
-      rowtab[rowbase[c] + r] = off;
-    }
-    for (int j = lane; j < n; j += 32) {
-      int x = j, off = 0;
-      for (int q = 0; q < mp.col.n; ++q) {
-        const int e = cd[mp.col.y[q]];
-        off += (x % e) * st[mp.col.y[q]];
-        x /= e;
+      for (int i = lane; i < ext; i += 32) {
+        int x = i, off = 0;
+        for (int q = 0; q < mm.n; ++q) {
+          const int e = cd[mm.y[q]];
+          off += (x % e) * st[mm.y[q]];
+          x /= e;
+        }
+        out[i] = off;
       }
-      coltab[colbase[c] + j] = off;
-    }
+    };
+    fill(mp.row, m, rowtab + rowbase[c]);
+    fill(mp.col, n, coltab + colbase[c]);
   }
 }
 
@@ -1291,6 +1297,11 @@ static void slice_layout(sht_tensor* T, const std::vector<int>& free_modes, cons
 
 int split_slices_default() { return 7; }
 
+void split_tile(int& m, int& n) {
+  m = kSplitM;
+  n = kSplitN;
+}
+
 void split_prepare(sht_plan* p, int S, cudaStream_t s) {
   split_layout(p, S, s);
   split_records(p, s);
@@ -1339,41 +1350,46 @@ void split_records(sht_plan* p, cudaStream_t s) {
   // the totals come back with the work list's counts
   const sht_tensor* C = p->C;
   const long long nc = C->nblocks;
-  PoolBuf drb(pool, std::max(nc, 1LL) * 8, s), dcb(pool, std::max(nc, 1LL) * 8, s);
-  PoolBuf rm(pool, std::max(nc, 1LL) * 8, s), rn(pool, std::max(nc, 1LL) * 8, s);
-  long long rtot = 0, ctot = 0;
-  if (nc > 0) {
-    k_round4<<<grid_for(nc, 256), 256, 0, s>>>(p->d_cm.as<int>(), p->d_cn.as<int>(), nc, rm.as<long long>(),
-                                               rn.as<long long>());
-    size_t tb = 0;
-    cub::DeviceScan::ExclusiveSum(nullptr, tb, rm.as<long long>(), drb.as<long long>(), (int)nc, s);
-    PoolBuf tmp(pool, tb, s);
-    cub::DeviceScan::ExclusiveSum(tmp.ptr, tb, rm.as<long long>(), drb.as<long long>(), (int)nc, s);
-    cub::DeviceScan::ExclusiveSum(tmp.ptr, tb, rn.as<long long>(), dcb.as<long long>(), (int)nc, s);
+  // (plans over small block grids have them, and the work list, from the pair counts)
+  if (!p->work_ready) {
+    p->sp_rowbase = PoolBuf(pool, std::max(nc, 1LL) * 8, s);
+    p->sp_colbase = PoolBuf(pool, std::max(nc, 1LL) * 8, s);
+    PoolBuf &drb = p->sp_rowbase, &dcb = p->sp_colbase;
+    PoolBuf rm(pool, std::max(nc, 1LL) * 8, s), rn(pool, std::max(nc, 1LL) * 8, s);
+    if (nc > 0) {
+      k_round4<<<grid_for(nc, 256), 256, 0, s>>>(p->d_cm.as<int>(), p->d_cn.as<int>(), nc, rm.as<long long>(),
+                                                 rn.as<long long>());
+      size_t tb = 0;
+      cub::DeviceScan::ExclusiveSum(nullptr, tb, rm.as<long long>(), drb.as<long long>(), (int)nc, s);
+      PoolBuf tmp(pool, tb, s);
+      cub::DeviceScan::ExclusiveSum(tmp.ptr, tb, rm.as<long long>(), drb.as<long long>(), (int)nc, s);
+      cub::DeviceScan::ExclusiveSum(tmp.ptr, tb, rn.as<long long>(), dcb.as<long long>(), (int)nc, s);
+    }
+    // work list: 128 x 32 tiles of every C block, heaviest blocks first, with per-tile and
+    // per-pair records so that the kernel reads each with one load
+    const DevSum extra[2] = {{drb.as<long long>() + nc - 1, rm.as<long long>() + nc - 1},
+                             {dcb.as<long long>() + nc - 1, rn.as<long long>() + nc - 1}};
+    long long h[2] = {0, 0};
+    // Many C blocks: order them by A row block (L2 reuse of the A slabs); the tiles are many per
+    // CTA, so the static striding stays balanced.  Few C blocks: heaviest first, for balance.
+    PoolBuf okey;
+    int obits = 0;
+    if (nc >= 16LL * p->ctx->num_sms) {
+      unsigned long long span = 1;
+      for (int t = 0; t < p->tmaps.row.n; ++t) span *= (unsigned long long)C->nblk[p->tmaps.row.y[t]];
+      int rbits = 0;
+      while (rbits < 62 && (1ull << rbits) < span) ++rbits;
+      obits = rbits + 1;
+      okey = PoolBuf(pool, nc * 8, s);
+      k_split_order_keys<<<grid_for(nc, 256), 256, 0, s>>>(C->d_ids.as<long long>(), nc, make_meta(C), p->tmaps.row,
+                                                           p->d_pstart.as<int>(), rbits, okey.as<unsigned long long>());
+      SHT_CUDA(cudaGetLastError());
+    }
+    device_work_list(p, kSplitM, kSplitN, false, s, extra, h, nc > 0 ? 2 : 0, okey.as<unsigned long long>(), obits);
+    p->sp_rtot = h[0];
+    p->sp_ctot = h[1];
   }
-  // work list: 128 x 32 tiles of every C block, heaviest blocks first, with per-tile and
-  // per-pair records so that the kernel reads each with one load
-  const DevSum extra[2] = {{drb.as<long long>() + nc - 1, rm.as<long long>() + nc - 1},
-                           {dcb.as<long long>() + nc - 1, rn.as<long long>() + nc - 1}};
-  long long h[2] = {0, 0};
-  // Many C blocks: order them by A row block (L2 reuse of the A slabs); the tiles are many per
-  // CTA, so the static striding stays balanced.  Few C blocks: heaviest first, for balance.
-  PoolBuf okey;
-  int obits = 0;
-  if (nc >= 16LL * p->ctx->num_sms) {
-    unsigned long long span = 1;
-    for (int t = 0; t < p->tmaps.row.n; ++t) span *= (unsigned long long)C->nblk[p->tmaps.row.y[t]];
-    int rbits = 0;
-    while (rbits < 62 && (1ull << rbits) < span) ++rbits;
-    obits = rbits + 1;
-    okey = PoolBuf(pool, nc * 8, s);
-    k_split_order_keys<<<grid_for(nc, 256), 256, 0, s>>>(C->d_ids.as<long long>(), nc, make_meta(C), p->tmaps.row,
-                                                         p->d_pstart.as<int>(), rbits, okey.as<unsigned long long>());
-    SHT_CUDA(cudaGetLastError());
-  }
-  device_work_list(p, kSplitM, kSplitN, false, s, extra, h, nc > 0 ? 2 : 0, okey.as<unsigned long long>(), obits);
-  rtot = h[0];
-  ctot = h[1];
+  const long long rtot = p->sp_rtot, ctot = p->sp_ctot;
   trace("split: work list", s);
   if (rtot >= (1LL << 31) || ctot >= (1LL << 31)) fail(SHT_ERR_UNSUPPORTED, "split mode: C row / column tables above 2^31");
   // a tile reads a full 128 rows / 32 columns: slack past the last block
@@ -1383,7 +1399,7 @@ void split_records(sht_plan* p, cudaStream_t s) {
   SHT_CUDA(cudaMemsetAsync(p->sp_coltab.ptr, 0, (ctot + kSplitN) * 4, s));
   if (nc > 0)
     k_split_offsets<<<(int)std::min<long long>((nc + 7) / 8, (long long)p->ctx->num_sms * 8), 256, 0, s>>>(
-        C->d_dims.as<int>(), nc, p->tmaps, drb.as<long long>(), dcb.as<long long>(), p->sp_rowtab.as<int>(),
+        C->d_dims.as<int>(), nc, p->tmaps, p->sp_rowbase.as<long long>(), p->sp_colbase.as<long long>(), p->sp_rowtab.as<int>(),
         p->sp_coltab.as<int>());
   trace("split: C offset tables", s);
   p->sp_items = PoolBuf(pool, std::max(p->bwork, 1LL) * sizeof(SplitItem), s);
@@ -1391,8 +1407,8 @@ void split_records(sht_plan* p, cudaStream_t s) {
   if (p->bwork > 0)
     k_split_items<<<grid_for(p->bwork, 256), 256, 0, s>>>(p->d_bwork.as<int4>(), (int)p->bwork, p->d_pstart.as<int>(),
                                                           p->C->d_offsets.as<long long>(), p->C->d_dims.as<int>(),
-                                                          p->tmaps, drb.as<long long>(), dcb.as<long long>(),
-                                                          p->sp_items.as<SplitItem>());
+                                                          p->tmaps, p->sp_rowbase.as<long long>(),
+                                                          p->sp_colbase.as<long long>(), p->sp_items.as<SplitItem>());
   if (p->npairs > 0)
     k_split_pairs<<<grid_for(p->npairs, 256), 256, 0, s>>>(
         p->d_pair_a.as<int>(), p->d_pair_b.as<int>(), p->npairs, p->sp_aoff,
