@@ -277,7 +277,7 @@ __global__ void k_count_missing(const long long* __restrict__ pc, long long np, 
 // what the host needs for its allocations; after one read-back, k_match_cells and k_match_pairs
 // write the pattern, the pairs and the work list.  The general path below takes about 45 launches
 // and reads for the same plan, two to five microseconds each: ijl,lk->ijk over 20 blocks per mode
-// (12,872 pairs), see the figures at match_build.
+// (12,872 pairs) planned in 330 us that way and in 85 us this way, host time and read-backs included.
 constexpr int kMatchCtas = 8, kMatchThreads = 1024;
 constexpr long long kMatchCells = 1 << 18;  // C's block grid
 constexpr int kMatchKeys = 512;             // contracted block grid: also the most pairs of one cell
@@ -595,10 +595,24 @@ struct MatchOut {
 __global__ void __launch_bounds__(256) k_match_cells(const __grid_constant__ MatchArgs g, MatchOut o) {
   __shared__ int kstart[kMatchKeys + 1];
   __shared__ unsigned long long bstart[kMatchBuckets];
-  match_kstart(g, kstart);
+  // even CTAs write the cells, odd CTAs place the pairs: two chains of dependent loads side by side
+  const int lane = threadIdx.x & 31, half = gridDim.x / 2, id = blockIdx.x / 2;
+  if (blockIdx.x & 1) {
+    match_kstart(g, kstart);
+    const int width = match_width(g);
+    for (int a = (id * 256 + threadIdx.x) / width; a < g.nA; a += half * 256 / width)
+      match_pairs_of(g, kstart, a, lane & (width - 1), width, [&](int b, int cell) {
+        // the old-block marks are not needed any more: the cells' cursors (from 0 or 1)
+        const int slot = g.pofs[cell] + (atomicAdd(&g.cold[cell], 2) >> 1);
+        o.tmp_a[slot] = a;
+        o.tmp_b[slot] = b;
+        o.tmp_c[slot] = g.cidx[cell];
+      });
+    return;
+  }
   {  // starts of the classes: four per thread
     __shared__ unsigned long long wsum[8];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int warp = threadIdx.x >> 5;
     unsigned long long v[4], t = 0;
     for (int i = 0; i < 4; ++i) {
       v[i] = t;
@@ -622,7 +636,7 @@ __global__ void __launch_bounds__(256) k_match_cells(const __grid_constant__ Mat
   }
   const bool by_row = g.split_m && *g.nocc >= g.many;
   __syncthreads();
-  const int lane = threadIdx.x & 31, gw = (blockIdx.x * 256 + threadIdx.x) >> 5, nw = gridDim.x * 8;
+  const int gw = (id * 256 + threadIdx.x) >> 5, nw = half * 8;
   for (int base = gw * 32; base < g.ncell; base += nw * 32) {
     const int cell = base + lane;
     const int ci = cell < g.ncell ? g.cidx[cell] : -1;
@@ -662,15 +676,6 @@ __global__ void __launch_bounds__(256) k_match_cells(const __grid_constant__ Mat
       }
     }
   }
-  const int width = match_width(g);
-  for (int a = (blockIdx.x * 256 + threadIdx.x) / width; a < g.nA; a += gridDim.x * 256 / width)
-    match_pairs_of(g, kstart, a, lane & (width - 1), width, [&](int b, int cell) {
-      // the old-block marks are not needed any more: the cells' cursors (from 0 or 1)
-      const int slot = g.pofs[cell] + (atomicAdd(&g.cold[cell], 2) >> 1);
-      o.tmp_a[slot] = a;
-      o.tmp_b[slot] = b;
-      o.tmp_c[slot] = g.cidx[cell];
-    });
 }
 
 // The pairs of each cell ranked by A block (no two have the same), with their records.
@@ -1001,7 +1006,7 @@ static bool match_finish(sht_plan* p, cudaStream_t s) {
   o.npairs = np;
   o.nblocks = nc;
   const long long warps = std::max<long long>((st->g.ncell + 31) / 32, st->g.nA);
-  k_match_cells<<<(unsigned)std::min<long long>((warps + 7) / 8, p->ctx->num_sms * 2LL), 256, 0, s>>>(st->g, o);
+  k_match_cells<<<2 * (unsigned)std::min<long long>((warps + 7) / 8, p->ctx->num_sms * 1LL), 256, 0, s>>>(st->g, o);
   if (np > 0)
     k_match_pairs<<<grid_for(np, 256), 256, 0, s>>>(
         o, rec_modes(A->order, p->maps.rowA, p->maps.colA), rec_modes(B->order, p->maps.colB, p->maps.rowB),
