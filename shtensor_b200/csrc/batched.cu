@@ -24,8 +24,8 @@ namespace sht {
 
 // resident CTAs of the persistent grid (the same for all instances: same shared memory, bounds)
 static int ring_grid(sht_ctx* ctx) {
-  static std::once_flag once;
-  std::call_once(once, [] {
+  static DeviceOnce once;
+  once.run(ctx->device, [] {
     for (auto* k : {k_tiles<kRingPlan>, k_tiles<kRingMulti>, k_tiles<kRingStack>}) {
       SHT_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(RingSmem)));
       int n = 0;
@@ -36,7 +36,9 @@ static int ring_grid(sht_ctx* ctx) {
   return ctx->num_sms * kRingCtas;
 }
 
-constexpr long long kRingWaitLimit = 1LL << 22;  // about a second
+// Polls of one wait, a microsecond each: above the time of any tile (the schedule warp waits for whole
+// tiles), so that only a fault runs it out.
+constexpr long long kRingWaitLimit = 1LL << 26;
 
 // addressing flags of an expression (tile_ring.cuh)
 static bool consecutive(const int* x, int n) {

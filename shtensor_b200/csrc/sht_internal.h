@@ -263,6 +263,13 @@ volatile int* ctx_error_word(sht_ctx* ctx);
 // the first device-side failure recorded since the last call (0 if none); clears it
 int ctx_take_error(sht_ctx* ctx);
 
+// f once per device (kernel attributes are a device's own), safe with several threads
+struct DeviceOnce {
+  std::once_flag flag[64];
+  template <class F>
+  void run(int device, F f) { std::call_once(flag[device & 63], f); }
+};
+
 // timing helpers
 double now_ms();
 // Phase trace of the host runtime, printed to stderr when SHT_TRACE=1 (the stream is

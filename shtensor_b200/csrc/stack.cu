@@ -447,9 +447,9 @@ static void (*const kStackDmma[6][4])(StagedArgs<double>) = {SHT_DMMA(1, 1), SHT
 static void (*const kStackFma[4][4])(StagedArgs<float>) = {SHT_FMA(1, 2), SHT_FMA(2, 4), SHT_FMA(4, 4), SHT_FMA(4, 8)};
 #undef SHT_FMA
 
-static void stack_setup() {
-  static std::once_flag once;
-  std::call_once(once, [] {
+static void stack_setup(int device) {
+  static DeviceOnce once;
+  once.run(device, [] {
     const int big = 96 * 1024;  // buffers and tables of the largest staged shape
     for (const auto& r : kStackDmma)
       for (auto* f : r) SHT_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
@@ -567,7 +567,7 @@ static void launch_stack(sht_kernel* k, const T* a, const T* b, T* c, long long 
   g.sc.beta_zero = std::memcmp(&be, zb, sizeof(T)) == 0;
   g.A = a; g.B = b; g.C = c;
   g.size_a = k->size_a; g.size_b = k->size_b; g.size_c = k->size_c;
-  stack_setup();
+  stack_setup(k->ctx->device);
   if (staged_fits(k, sizeof(T))) launch_staged_op(k, g, nb_ops, s);
   else launch_large(k, g, nb_ops, s);
 }
