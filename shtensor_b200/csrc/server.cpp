@@ -71,6 +71,9 @@ struct Request {
   int deferrals = 0;
   bool waiting_memory = false;  // deferred; retried after the next retired launch
   int64_t deferred_at = -1;     // retired-launch count when it was deferred
+  // out of pool memory with nothing else active, while callers may still return finished requests'
+  // tensors: since when, and when it is planned again
+  Clock::time_point oom_since{}, retry_at{};
   int64_t npairs = 0;
   double flops = 0.0;
   int form = SHT_MODE_BATCHED_FP64;  // the form it was planned in
@@ -120,6 +123,8 @@ struct sht_server {
   int64_t next_id = 1;
   bool stop = false, stop_planners = false;
   int completions = 0;  // launch completions seen by the waiter, not yet handled
+  int64_t uncollected = 0;         // finished requests that no wait has returned yet
+  Clock::time_point last_collect{};  // the last wait that returned one
   // statistics since the last reset
   int64_t submitted = 0, completed = 0, failed = 0, batches = 0, batched_reqs = 0, deferrals = 0;
   int max_active_seen = 0;
@@ -153,6 +158,7 @@ struct sht_server {
   bool admit();
   bool launch();
   void defer(Request& r);
+  bool memory_may_return(Request& r);
   void finish(const ReqPtr& r, sht_status st, const std::string& msg, Clock::time_point t);
   int active() const {
     int n = (int)ready.size() + (int)planning.size();
@@ -199,6 +205,7 @@ void sht_server::finish(const ReqPtr& r, sht_status st, const std::string& msg, 
   r->msg = msg;
   r->t_done = t;
   r->finished = true;
+  ++uncollected;
   if (st == SHT_OK) {
     ++completed;
     latencies.push_back(ms_between(r->t_submit, t));
@@ -258,6 +265,19 @@ void sht_server::defer(Request& r) {
   ++deferrals;
 }
 
+// Whether a request that found no memory with nothing else active should be planned again: finished
+// requests' tensors are their callers' to free, which takes them a moment after (or before) the wait
+// that returns the request.  It gives up a second after its first such try, or after the last
+// collected request if that was later, so that a caller waiting for this very request gets its
+// failure.
+bool sht_server::memory_may_return(Request& r) {
+  const Clock::time_point now = Clock::now();
+  if (r.oom_since == Clock::time_point{}) r.oom_since = now;
+  std::lock_guard<std::mutex> lk(mu);
+  if (uncollected == 0 && now - last_collect > std::chrono::milliseconds(100)) return false;
+  return now - std::max(r.oom_since, last_collect) < std::chrono::seconds(1);
+}
+
 // Take the planners' results: planned requests become ready; a plan that ran out of pool
 // memory while other requests hold memory goes back to the queue; other failures finish.
 bool sht_server::collect() {
@@ -273,6 +293,12 @@ bool sht_server::collect() {
       ready.push_back(std::move(r));
     } else if (r->plan_status == SHT_ERR_OOM && active() > 0) {
       strace("defer request %lld (out of pool memory)", (long long)r->id);
+      r->oom_since = Clock::time_point{};
+      defer(*r);
+      insert_by_id(queued, std::move(r));
+    } else if (r->plan_status == SHT_ERR_OOM && memory_may_return(*r)) {
+      strace("retry request %lld (finished requests hold memory)", (long long)r->id);
+      r->retry_at = Clock::now() + std::chrono::milliseconds(3);
       defer(*r);
       insert_by_id(queued, std::move(r));
     } else {
@@ -312,6 +338,7 @@ bool sht_server::admit() {
     // a deferred request waits for a retired launch to return memory; later requests keep
     // their order behind it
     if (others && r.waiting_memory && r.deferred_at == retired_launches) break;
+    if (r.retry_at > Clock::now()) break;
     // requests with the planners may not have taken their memory yet: count their estimates
     size_t planning_bytes = 0;
     for (const ReqPtr& o : planning) planning_bytes += estimate_bytes(*o, mode);
@@ -533,7 +560,7 @@ void sht_server::loop() {
     // idle: sleep until a submit, a planned request, a completion or stop; the
     // timeout bounds the wait for a launch whose callback cannot arrive (a failed stream)
     if (incoming.empty() && planned.empty())
-      wake.wait_for(lk, std::chrono::milliseconds(running.empty() ? 50 : 2),
+      wake.wait_for(lk, std::chrono::milliseconds(running.empty() && queued.empty() ? 50 : 2),
                     [&] { return stop || !incoming.empty() || !planned.empty() || completions > 0; });
     completions = 0;
   }
@@ -651,6 +678,8 @@ sht_status sht_server_wait(sht_server* srv, int64_t request_id, double timeout_s
       fail(SHT_ERR_TIMEOUT, "request " + std::to_string(request_id) + " still pending");
     }
     srv->table.erase(it);
+    --srv->uncollected;
+    srv->last_collect = Clock::now();
   });
   if (st != SHT_OK) return st;
   if (rep) {
