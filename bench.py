@@ -717,10 +717,14 @@ def run_ours(args):
     cpu = None
     if rank == 0 and world == 1 and not args.no_cpu:
         ncores = os.cpu_count() or 1
-        legs = {"reference_openmp": cpu_leg(w, args.cpu_sample_seconds / args.cpu_runs, ncores, True, args.cpu_runs),
-                "reference_1thread": cpu_leg(w, 2.0, 1, True, args.cpu_runs),
-                "xmm_restatement_1thread": cpu_leg(w, 2.0, 1, False, args.cpu_runs)}
-        cpu = dict(legs["reference_openmp"])
+        import oracle
+        ref = oracle.ref_lib() is not None  # without the reference's sources: the restatement alone
+        main_leg = "reference_openmp" if ref else "xmm_restatement_openmp"
+        legs = {main_leg: cpu_leg(w, args.cpu_sample_seconds / args.cpu_runs, ncores, ref, args.cpu_runs)}
+        if ref:
+            legs["reference_1thread"] = cpu_leg(w, 2.0, 1, True, args.cpu_runs)
+        legs["xmm_restatement_1thread"] = cpu_leg(w, 2.0, 1, False, args.cpu_runs)
+        cpu = dict(legs[main_leg])
         cpu["legs"] = legs
 
     del A, B, Cd
