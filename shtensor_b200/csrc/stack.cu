@@ -11,6 +11,7 @@
 //   * larger FP64 blocks: the ring tile kernel (tile_ring.cuh), one pair per C block;
 //   * larger FP32 blocks: the gathering tile (tile_core.cuh).
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 
 #include "contract.h"
@@ -382,9 +383,10 @@ static void staged_wavefronts(const StagedModes& rows, const StagedModes& ks, in
 }
 
 // FP32 register tile and lanes along rows: the least issue slots over the op's groups (products,
-// operand and table reads per k).
+// operand and table reads per k).  With few ops (an SM or more for each) the op's own time counts:
+// its groups run at once on up to kStagedWarpsMax warps, each k waiting about 40 cycles for its reads.
 struct FmaShape { int rm, cn, lr; };
-static FmaShape pick_fma_shape(int m, int n) {
+static FmaShape pick_fma_shape(int m, int n, bool few) {
   static const int tiles[][2] = {{1, 2}, {2, 4}, {4, 4}, {4, 8}};
   FmaShape best{4, 8, 32};
   double bc = 1e300;
@@ -392,7 +394,8 @@ static FmaShape pick_fma_shape(int m, int n) {
     for (int lr = 32; lr >= 8; lr /= 2) {
       const int rt = t[0] * lr, ct = t[1] * (32 / lr);
       const double groups = (double)((m + rt - 1) / rt) * (double)((n + ct - 1) / ct);
-      const double c = groups * (t[0] * t[1] + 1.5 * (t[0] + t[1]) + 6);
+      const double k = t[0] * t[1] + 1.5 * (t[0] + t[1]) + 6;
+      const double c = few ? std::ceil(groups / kStagedWarpsMax) * (k + 40) : groups * k;
       if (c < bc) { bc = c; best = {t[0], t[1], lr}; }
     }
   return best;
@@ -409,7 +412,7 @@ void stack_prepare(sht_kernel* k) {
   const StagedModes cb = staged_modes(k->maps.colB, k->sb), kb = staged_modes(k->maps.rowB, k->sb);
   const int m = (int)k->m, n = (int)k->n, K = (int)k->k;
   // FP32 columns are the same for whole rows of lanes: only A's reads spread over the banks
-  const int lr = f64 ? 8 : pick_fma_shape(m, n).lr;
+  const int lr = f64 ? 8 : pick_fma_shape(m, n, false).lr;
   int w[2] = {0, 0};
   staged_wavefronts(ra, ka, m, K, f64, lr, w);
   if (f64) staged_wavefronts(cb, kb, n, K, f64, 8, w);
@@ -424,8 +427,9 @@ static bool staged_fits(const sht_kernel* k, size_t es) {
 }
 
 template <typename T, class Kernel>
-static void launch_staged(sht_kernel* k, const StagedArgs<T>& s, int groups, Kernel kernel, cudaStream_t st) {
-  const int warps = std::min(groups, kStagedWarpsMax);
+static void launch_staged(sht_kernel* k, const StagedArgs<T>& s, int groups, bool few, Kernel kernel, cudaStream_t st) {
+  // a warp per group of the block; more where the copies would take a thread many turns
+  const int warps = std::min(std::max(groups, few ? (s.abytes + s.bbytes) / 1024 : 0), kStagedWarpsMax);
   const size_t smem = (((size_t)2 * (s.mp + s.np + s.kp) * 4 + 127) & ~(size_t)127) + 2 * (size_t)(s.abytes + s.bbytes);
   // resident CTAs by shared memory and by threads (a persistent wave; ops are strided over it)
   const long long per_sm = std::max<long long>(1, std::min<long long>({32, 227 * 1024 / (long long)(smem + 1024), 32 / warps}));
@@ -458,20 +462,34 @@ static void stack_setup(int device) {
   });
 }
 
+// An SM for each op: a call then takes the latency of one op, not its share of issue slots.  Measured
+// with the event overhead of a lone call (11.6 us): FP32 ik,kj->ij 63x51 by 51x10, 13 ops: 20.5 us
+// with the issue-bound shape, 13.9 us so; FP64 ikl,ljk->ij 5x16x9, 117 ops: 17.3 and 11.9.
+static bool few_ops(const sht_kernel* k, long long nb_ops) { return nb_ops <= k->ctx->num_sms; }
 static void launch_staged_op(sht_kernel* k, const StackArgs<double>& g, long long nb_ops, cudaStream_t st) {
-  // the smallest tile that takes the block's rows and columns at once, up to 32 x 16
-  const int ri = k->m <= 8 ? 0 : k->m <= 16 ? 1 : 2, ci = k->n <= 8 ? 0 : 1, rt = 8 << ri, ct = 8 << ci;
+  // the smallest tile that takes the block's rows and columns at once, up to 32 x 16; with few ops the
+  // smallest whose groups a CTA's warps take at once
+  const bool few = few_ops(k, nb_ops);
+  int ri = k->m <= 8 ? 0 : k->m <= 16 ? 1 : 2, ci = k->n <= 8 ? 0 : 1;
+  for (int t = 0, end = few ? 2 * ri + ci : 0; t < end; ++t)
+    if (((k->m - 1) / (8 << t / 2) + 1) * ((k->n - 1) / (8 << t % 2) + 1) <= kStagedWarpsMax) {
+      ri = t / 2;
+      ci = t % 2;
+      break;
+    }
+  const int rt = 8 << ri, ct = 8 << ci;
   const StagedArgs<double> s = staged_args(k, g, nb_ops, rt, ct);
-  launch_staged(k, s, (s.mp / rt) * (s.np / ct), kStackDmma[2 * ri + ci][(s.sc.alpha != 1.0 ? 2 : 0) + (k->swizzle ? 1 : 0)],
+  launch_staged(k, s, (s.mp / rt) * (s.np / ct), few, kStackDmma[2 * ri + ci][(s.sc.alpha != 1.0 ? 2 : 0) + (k->swizzle ? 1 : 0)],
                 st);
 }
 static void launch_staged_op(sht_kernel* k, const StackArgs<float>& g, long long nb_ops, cudaStream_t st) {
-  const FmaShape f = pick_fma_shape((int)k->m, (int)k->n);
+  const bool few = few_ops(k, nb_ops);
+  const FmaShape f = pick_fma_shape((int)k->m, (int)k->n, few);
   const int rt = f.rm * f.lr, ct = f.cn * (32 / f.lr);
   StagedArgs<float> s = staged_args(k, g, nb_ops, rt, ct);
   s.lr = f.lr;
   const int tile = f.rm == 1 ? 0 : f.rm == 2 ? 1 : f.cn == 4 ? 2 : 3;
-  launch_staged(k, s, (s.mp / rt) * (s.np / ct), kStackFma[tile][(s.sc.alpha != 1.0f ? 2 : 0) + (k->swizzle ? 1 : 0)], st);
+  launch_staged(k, s, (s.mp / rt) * (s.np / ct), few, kStackFma[tile][(s.sc.alpha != 1.0f ? 2 : 0) + (k->swizzle ? 1 : 0)], st);
 }
 
 // ------------------------------------------------------------------ larger blocks
