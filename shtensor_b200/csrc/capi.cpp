@@ -44,6 +44,21 @@ struct LaneLease {
   LaneLease& operator=(const LaneLease&) = delete;
 };
 
+// Leaving a contraction by an error: what its plan queued on the lane stream ps (C's grown index and
+// blocks among it) is complete, and the tensors' memory is released against the caller's stream s
+// again, whose earlier work may still read it.
+struct PlanGuard {
+  sht_plan* p;
+  cudaStream_t ps, s;
+  bool done = false;
+  ~PlanGuard() {
+    if (done) return;
+    cudaStreamSynchronize(ps);
+    p->index_pending = false;
+    plan_touch(p, s);
+  }
+};
+
 // Split form of sht_contract with the slicer overlapped: the slices depend on the patterns and
 // values of A and B only, so they run on the caller's stream s while the pair list, result
 // pattern and records are built on a second stream, which first waits for the work already
@@ -52,6 +67,7 @@ static void contract_split(sht_plan* p, double alpha, double beta, cudaStream_t 
   sht_ctx* ctx = p->ctx;
   LaneLease lane(ctx);
   const cudaStream_t ps = lane.lane.stream;
+  PlanGuard guard{p, ps, s};
   SHT_CUDA(cudaEventRecord(lane.lane.start, s));
   p->caller_event = lane.lane.start;
   // without screening the counting kernel of the plan goes ahead of the slicer, whose CTAs fill the SMs
@@ -91,6 +107,7 @@ static void contract_split(sht_plan* p, double alpha, double beta, cudaStream_t 
   split_launch(p, sparse_args(p, alpha, beta), s);
   trace("contract: split kernel launched", s);
   plan_settle(p, ps);
+  guard.done = true;
 }
 
 // A bounded wait of an earlier launch on this context ran out: report it at this call.
@@ -113,6 +130,7 @@ static void contract_fp64(sht_plan* p, double alpha, double beta, cudaStream_t s
   sht_ctx* ctx = p->ctx;
   LaneLease lane(ctx);
   const cudaStream_t ps = lane.lane.stream;
+  PlanGuard guard{p, ps, s};
   SHT_CUDA(cudaEventRecord(lane.lane.start, s));
   p->caller_event = lane.lane.start;
   if (p->eps > 0.0) SHT_CUDA(cudaStreamWaitEvent(ps, lane.lane.start, 0));
@@ -132,6 +150,7 @@ static void contract_fp64(sht_plan* p, double alpha, double beta, cudaStream_t s
   ring_launch(p, sparse_args(p, alpha, beta), s);
   trace("contract: tile kernel launched", s);
   plan_settle(p, ps);
+  guard.done = true;
 }
 
 volatile int* ctx_error_word(sht_ctx* ctx) {
