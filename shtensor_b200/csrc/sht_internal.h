@@ -209,11 +209,11 @@ struct sht_tensor {
   std::vector<std::vector<int>> bs;
   std::vector<int> nblk;
   std::vector<int64_t> gstride;
-  // host index (authoritative unless host_stale)
+  // host index (authoritative unless host_stale; read back under hmu: tensor_sync_host)
   std::vector<int64_t> ids, offsets, rows;
-  bool host_stale = false;
-  bool stale_unmarked = false;  // host_stale, and known to hold no filtered id
-  bool has_marked = false;  // the host index holds filtered (negative) ids
+  std::atomic<bool> host_stale{false};
+  std::atomic<bool> stale_unmarked{false};  // host_stale, and known to hold no filtered id
+  std::atomic<bool> has_marked{false};  // the host index holds filtered (negative) ids
   // per-block extents and block-grid coordinates (nblocks x order each) of the host index,
   // computed on first use after the host index changes (tensor_host_dims, tensor_host_coords)
   std::vector<int> hdims, hcoords;

@@ -221,13 +221,13 @@ void tensor_touch(sht_tensor* t, cudaStream_t s) {
   for (PoolBuf* b : {&t->d_bsizes, &t->d_bstart, &t->d_ids, &t->d_offsets, &t->d_dims, &t->d_data}) b->use_on(s);
 }
 
-// Pull the device index back to the host mirror when a device-side operation rebuilt it.
+// Pull the device index back to the host mirror when a device-side operation rebuilt it.  Any thread
+// that reads a tensor may be the one to do it (a server's loop and the tensor's owner at once).
 void tensor_sync_host(sht_tensor* t, cudaStream_t s) {
   if (!t->host_stale) return;
-  {
-    std::lock_guard<std::mutex> lk(t->hmu);
-    t->hdims_valid = false;
-  }
+  std::lock_guard<std::mutex> lk(t->hmu);
+  if (!t->host_stale) return;  // another thread has done it meanwhile
+  t->hdims_valid = false;
   t->ids.resize(t->nblocks);
   t->offsets.resize(t->nblocks);
   if (t->nblocks) {

@@ -92,3 +92,29 @@ def test_split_growth_orders_after_earlier_work(ctx):
         s.synchronize()
         assert np.array_equal(c.get_sparse_info()[0], w2.C.ids)
         assert np.linalg.norm(c.download() - w2.C.data) <= 1e-12 * np.linalg.norm(w2.C.data)
+
+
+def test_server_and_owner_read_a_grown_index_at_once(ctx):
+    # a grown tensor is submitted as an operand, and its owner reads its index while the server's loop
+    # reads the same index back for planning
+    rng = np.random.default_rng(8)
+    n, k = [2] * 100, [3]
+    A = W.build_tensor(rng, [n, k], lambda c: np.ones(len(c[0]), bool), None, "normal")
+    B = W.build_tensor(rng, [k, n], lambda c: np.ones(len(c[0]), bool), None, "normal")
+    V = W.build_tensor(rng, [n, k], lambda c: np.ones(len(c[0]), bool), None, "normal")
+    a, b, v = dev(ctx, A), dev(ctx, B), dev(ctx, V)
+    w1 = oracle.contract(EXPR, 1.0, host(A), host(B), 0.0, host(W.empty_tensor([n, n])))
+    w2 = oracle.contract(EXPR, 1.0, oracle.HostTensor([n, n], w1.C.ids, w1.C.offsets, w1.C.data), host(V), 0.0,
+                         host(W.empty_tensor([n, k])))
+    ds = [dev(ctx, W.empty_tensor([n, n])) for _ in range(40)]
+    for d in ds:
+        sht.contract(ctx, EXPR, 1.0, a, b, 0.0, d)
+    ctx.stream_sync()
+    with sht.Server(ctx) as srv:
+        for d in ds:
+            e = dev(ctx, W.empty_tensor([n, k]))
+            rid = srv.submit(EXPR, 1.0, d, v, 0.0, e)
+            ids, offs, _ = d.get_sparse_info()
+            assert np.array_equal(ids, w1.C.ids) and np.array_equal(offs, w1.C.offsets)
+            srv.wait(rid, 60)
+            assert bits_equal(e.download(), w2.C.data)
