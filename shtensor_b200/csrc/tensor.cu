@@ -227,6 +227,9 @@ void tensor_sync_host(sht_tensor* t, cudaStream_t s) {
   if (!t->host_stale) return;
   std::lock_guard<std::mutex> lk(t->hmu);
   if (!t->host_stale) return;  // another thread has done it meanwhile
+  // a contraction that grew the index returned with it complete: it need not wait for the caller's
+  // stream, which may still compute the tensor's values
+  if (t->stale_unmarked) s = t->ctx->stage_stream;
   t->hdims_valid = false;
   t->ids.resize(t->nblocks);
   t->offsets.resize(t->nblocks);

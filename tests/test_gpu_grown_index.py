@@ -118,3 +118,27 @@ def test_server_and_owner_read_a_grown_index_at_once(ctx):
             assert np.array_equal(ids, w1.C.ids) and np.array_equal(offs, w1.C.offsets)
             srv.wait(rid, 60)
             assert bits_equal(e.download(), w2.C.data)
+
+
+@pytest.mark.parametrize("mode", [sht.Mode.PLAIN_FP64, sht.Mode.BATCHED_FP64])
+def test_grown_operand_does_not_wait_for_the_stream(ctx, mode):
+    # D = A B grows D; E = D A is then planned and queued while the stream is still busy
+    import torch
+    rng = np.random.default_rng(9)
+    A = full(rng, 6, 6)
+    a = dev(ctx, A)
+    w1 = oracle.contract(EXPR, 1.0, host(A), host(A), 0.0, host(W.empty_tensor(A.block_sizes)))
+    w2 = oracle.contract(EXPR, 1.0, oracle.HostTensor(A.block_sizes, w1.C.ids, w1.C.offsets, w1.C.data), host(A), 0.0,
+                         host(W.empty_tensor(A.block_sizes)))
+    s = torch.cuda.Stream()
+    for cycles in (1000, 4 * BUSY):  # the first turn loads the kernels
+        d, e = dev(ctx, W.empty_tensor(A.block_sizes)), dev(ctx, W.empty_tensor(A.block_sizes))
+        sht.contract(ctx, EXPR, 1.0, a, a, 0.0, d, mode=mode, stream=s)
+        s.synchronize()
+        with torch.cuda.stream(s):
+            torch.cuda._sleep(cycles)
+        sht.contract(ctx, EXPR, 1.0, d, a, 0.0, e, mode=mode, stream=s)
+        busy = not s.query()
+        s.synchronize()
+        assert bits_equal(e.download(), w2.C.data)
+    assert busy
