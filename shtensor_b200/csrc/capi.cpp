@@ -518,6 +518,8 @@ sht_status sht_plan_create(sht_ctx* ctx, const char* expr, sht_tensor* A, sht_te
     need(norm >= SHT_NORM_FROBENIUS && norm <= SHT_NORM_FROBENIUS_REFCOMPAT, "unknown norm");
     std::unique_ptr<sht_plan> p(plan_create(ctx, expr, A, B, C, eps, norm, mode, as_stream(stream)));
     prepare_mode(p.get(), as_stream(stream));
+    // every list is complete: the plan may be executed on another stream
+    SHT_CUDA(cudaStreamSynchronize(as_stream(stream)));
     *out = p.release();
   });
 }

@@ -1071,7 +1071,7 @@ sht_plan* plan_create(sht_ctx* ctx, const std::string& expr, sht_tensor* A, sht_
                       double eps, sht_norm norm, sht_mode mode, cudaStream_t s) {
   std::unique_ptr<sht_plan> p(plan_init(ctx, expr, A, B, C, eps, norm, mode, s));
   plan_build(p.get(), s);
-  // the pair list can be read back on another stream, and C's index by any later call
+  // C's index is complete for any later call; callers order what they queue next on s themselves
   SHT_CUDA(cudaStreamSynchronize(s));
   p->index_pending = false;
   return p.release();
