@@ -179,15 +179,17 @@ sht_status sht_set_split_slices(sht_ctx* ctx, int slices);
 /* Every form is asynchronous: sht_contract and sht_plan_execute return once the work is queued on
  * `stream`.  The waits inside the contraction kernels (and of sht_kernel_call's for large blocks)
  * are bounded; a wait that runs out (a hardware or scheduling fault) leaves C undefined and records
- * SHT_ERR_TIMEOUT on the context.  The next contraction, execute or stack call on the context
- * reports it (without queueing its own work), and sht_stream_sync reports it after the stream's
+ * SHT_ERR_TIMEOUT on the context.  The next sht_contract, sht_plan_execute, sht_plan_execute_graph
+ * or sht_kernel_call on the context reports it (without queueing its own work), and sht_stream_sync reports it after the stream's
  * work is done.  Non-finite inputs of the split form are not an error: such an execute is computed
  * by the FP64 tiles, with IEEE propagation as in the FP64 forms. */
 /* waits for the work queued on `stream`, then returns (and clears) the first failure recorded
  * by this context's device work, if any */
 sht_status sht_stream_sync(sht_ctx* ctx, void* stream);
-/* diagnostic: polls of one device pipeline wait of the split kernel before the launch gives up
- * (0 = the default, about a second); waits for work already issued keep their own bound */
+/* diagnostic: polls of one wait inside the contraction kernels before the launch gives up.  0 = the
+ * default: about a second for the split kernel, about a minute for the FP64 tile kernel, whose waits
+ * can last as long as a tile.  Waits for work already issued keep their own bound, and a graph
+ * captured by sht_plan_execute_graph keeps the limit it was captured with. */
 sht_status sht_set_wait_limit(sht_ctx* ctx, int64_t polls);
 
 /* ---- diagnostics ---- */

@@ -228,11 +228,11 @@ class Context:
 
     def stream_sync(self, stream=None):
         """Wait for the work queued on `stream` and raise the first failure this context's
-        device work recorded (a split launch whose bounded wait ran out)."""
+        device work recorded (a launch whose bounded wait ran out)."""
         _check(lib().sht_stream_sync(self._h, _stream(stream)))
 
     def set_wait_limit(self, polls: int):
-        """Diagnostic: polls of one split-kernel pipeline wait before the launch gives up (0 =
+        """Diagnostic: polls of one wait inside a contraction kernel before the launch gives up (0 =
         default)."""
         _check(lib().sht_set_wait_limit(self._h, int(polls)))
 

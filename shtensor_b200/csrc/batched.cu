@@ -36,9 +36,9 @@ static int ring_grid(sht_ctx* ctx) {
   return ctx->num_sms * kRingCtas;
 }
 
-// Polls of one wait, a microsecond each: above the time of any tile (the schedule warp waits for whole
-// tiles), so that only a fault runs it out.
-constexpr long long kRingWaitLimit = 1LL << 26;
+// Polls of one wait, up to a microsecond each: above the time of any tile (the schedule warp waits for
+// whole tiles), so that only a fault runs it out.  sht_set_wait_limit replaces it.
+static long long ring_wait_limit(const sht_ctx* ctx) { return ctx->wait_limit > 0 ? ctx->wait_limit : 1LL << 26; }
 
 // addressing flags of an expression (tile_ring.cuh)
 static bool consecutive(const int* x, int n) {
@@ -345,7 +345,7 @@ static RingArgs ring_args(sht_plan* p, const SparseArgs& g) {
   r.nwork = (int)((bb == one) ? p->bwork_touched : p->bwork);
   r.counter = p->d_counter.as<unsigned>();
   r.err = ctx_error_word(p->ctx);
-  r.wait_limit = kRingWaitLimit;
+  r.wait_limit = ring_wait_limit(p->ctx);
   return r;
 }
 
@@ -408,7 +408,7 @@ void ring_stack(sht_ctx* ctx, const SparseArgs& a, const PairRec& rec, const int
   r.tiles_per_op = (int)tiles;
   r.nwork = (int)(tiles * nb_ops);
   r.err = ctx_error_word(ctx);
-  r.wait_limit = kRingWaitLimit;
+  r.wait_limit = ring_wait_limit(ctx);
   const int grid = std::min(ring_grid(ctx), r.nwork);
   k_tiles<kRingStack><<<grid, kRingThreads, sizeof(RingSmem), s>>>(r);
   SHT_CUDA(cudaGetLastError());

@@ -537,6 +537,7 @@ sht_status sht_plan_execute_graph(sht_plan* p, double alpha, double beta, void* 
     need(p, "null plan");
     cudaStream_t s = as_stream(stream);
     if (!s) fail(SHT_ERR_INVALID, "graph replay needs a non-default stream");
+    raise_pending(p->ctx);
     if (p->graph_exec && (p->graph_alpha != alpha || p->graph_beta != beta)) {
       cudaGraphExecDestroy(p->graph_exec);
       cudaGraphDestroy(p->graph);
@@ -678,8 +679,8 @@ sht_status sht_stream_sync(sht_ctx* ctx, void* stream) {
     need(ctx, "null context");
     SHT_CUDA(cudaStreamSynchronize(as_stream(stream)));
     if (const int e = ctx_take_error(ctx))
-      fail((sht_status)e, "a split-precision launch on this context failed: a bounded wait on the tensor cores "
-                          "expired (its result is undefined)");
+      fail((sht_status)e, "a launch on this context failed: a bounded wait of its kernel expired (its result is "
+                          "undefined)");
   });
 }
 

@@ -227,11 +227,11 @@ bool sht_server::retire() {
     const Clock::time_point t = Clock::now();
     sht_status st = q == cudaSuccess ? SHT_OK : SHT_ERR_CUDA;
     std::string msg = q == cudaSuccess ? "" : std::string("serving launch failed: ") + cudaGetErrorString(q);
-    // a split launch whose bounded wait ran out recorded it on the context's error word
+    // a launch whose bounded wait ran out recorded it on the context's error word
     if (st == SHT_OK) {
       if (const int e = sht::ctx_take_error(ctx)) {
         st = (sht_status)e;
-        msg = "serving launch failed: a bounded wait on the tensor cores expired";
+        msg = "serving launch failed: a bounded wait of its kernel expired";
       }
     }
     if (q != cudaSuccess) (void)cudaGetLastError();

@@ -176,7 +176,7 @@ struct sht_ctx {
   std::map<std::string, int> tuned;     // autotuner choices: size-class key -> tile id
   int split_slices = 0;                 // INT8 slices per operand in split mode (0 = default)
   long long wait_limit = 0;             // polls of a device pipeline wait (0 = default)
-  // Error word of device work (a bounded wait of the split kernel that ran out): host memory
+  // Error word of device work (a bounded wait of a contraction kernel that ran out): host memory
   // mapped into the device, written by a kernel only on failure and read by the host without
   // a synchronization; sticky until reported (created on first use)
   int* err_host = nullptr;
