@@ -422,13 +422,17 @@ void ring_launch(sht_plan* p, const SparseArgs& g, cudaStream_t s) {
 // ------------------------------------------------------------------ autotuner
 // For every size class with work, time each tile shape on a sample of the class's C blocks
 // (written to a scratch copy, never to C) and keep the fastest.  Choices persist in the
-// context and, when a file is given, in a "key shape" text file keyed by GPU name.
+// context and, when a file is given, in a "key shape" text file keyed by GPU name and set of shapes.
 void autotune(sht_plan* p, const char* cache_file, cudaStream_t s) {
   sht_ctx* ctx = p->ctx;
   cudaDeviceProp prop;
   SHT_CUDA(cudaGetDeviceProperties(&prop, ctx->device));
   std::string gpu = prop.name;
   std::replace(gpu.begin(), gpu.end(), ' ', '_');
+  // a choice is a number in a set of tile shapes: lines under the bare GPU name were written for
+  // another set (64x64, 128x32, 32x128, 128x16)
+  for (int sh = 0; sh < kRingShapes; ++sh)
+    gpu += (sh ? "," : ":") + std::to_string(ring_tm(sh)) + "x" + std::to_string(ring_tn(sh));
   if (cache_file) {
     std::ifstream in(cache_file);
     std::string g, k;
