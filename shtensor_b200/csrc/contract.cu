@@ -1368,7 +1368,9 @@ SparseArgs sparse_args(sht_plan* p, double alpha, double beta) {
 
 void plan_touch(sht_plan* p, cudaStream_t s) {
   for (sht_tensor* t : {p->A, p->B, p->C}) tensor_touch(t, s);
-  for (PoolBuf* b : {&p->d_pair_a, &p->d_pair_b, &p->d_recs, &p->d_pstart, &p->d_bwork, &p->d_counter}) b->use_on(s);
+  for (PoolBuf* b : {&p->d_pair_a, &p->d_pair_b, &p->d_recs, &p->d_pstart, &p->d_bwork, &p->d_counter, &p->lin_a,
+                     &p->lin_b})
+    b->use_on(s);
   for (PoolBuf* b : {&p->sp_a, &p->sp_b, &p->sp_ae, &p->sp_be, &p->sp_bsc, &p->sp_meta, &p->sp_items, &p->sp_pairs,
                      &p->sp_rowtab, &p->sp_coltab, &p->sp_rowbase, &p->sp_colbase})
     b->use_on(s);

@@ -30,6 +30,7 @@ struct sht_plan {
   sht::PoolBuf d_cm, d_cn, d_cksum; // per C block: rows, columns, sum of the pairs' k
   sht::PoolBuf d_bwork;             // int4 per tile (ring_item; split plans: (C block, tile, ., .))
   sht::PoolBuf d_counter;           // work counter of the persistent FP64 kernel
+  sht::PoolBuf lin_a, lin_b;        // operands in the order that kernel reads (linear.cu), when they need it
   long long bwork = 0, bwork_touched = 0;
   // split path: INT8 slices (K-major rows), row / column exponents, error words
   sht::PoolBuf sp_a, sp_b, sp_ae, sp_be;
@@ -98,13 +99,17 @@ void device_work_list(sht_plan* p, int fixed_tm, int fixed_tn, bool per_class, c
                       const DevSum* extra = nullptr, long long* extra_out = nullptr, int nextra = 0,
                       const unsigned long long* order_key = nullptr, int order_bits = 0);
 void plan_execute(sht_plan* p, double alpha, double beta, cudaStream_t s);
-// the FP64 forms: work list and counter, then the persistent kernel
+// the FP64 forms: work list and counter, then (ring_launch) the operands' copy and the persistent kernel
 void ring_prepare(sht_plan* p, cudaStream_t s);
 void ring_launch(sht_plan* p, const SparseArgs& g, cudaStream_t s);
 // a stack of equal block triples (Kernel<double>::call): one pair per C block, its extents and strides
 // in rec, its block extents in dA / dB / dC
 void ring_stack(sht_ctx* ctx, const SparseArgs& a, const PairRec& rec, const int* dA, const int* dB, const int* dC,
                 long long size_a, long long size_b, long long size_c, int m, int n, long long nb_ops, cudaStream_t s);
+// operands whose modes lie apart (linear.cu): scratch and pair records at plan time, the copy per execute
+bool modes_consecutive(const int* x, int n);
+void linear_prepare(sht_plan* p, cudaStream_t s);
+void linear_execute(sht_plan* p, cudaStream_t s);
 void autotune(sht_plan* p, const char* cache_file, cudaStream_t s);
 size_t batched_desc_bytes();
 int batched_ctas_per_sm(sht_ctx* ctx);

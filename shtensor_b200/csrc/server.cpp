@@ -424,6 +424,7 @@ void sht_server::planner(int index) {
         r->kind = -1;
         r->plan.reset(sht::plan_create(ctx, r->expr, r->A, r->B, r->C, r->eps, r->norm, SHT_MODE_BATCHED_FP64, s));
         sht::ring_prepare(r->plan.get(), s);
+        if (!sht::sparse_args(r->plan.get(), r->alpha, r->beta).sc.alpha_zero) sht::linear_execute(r->plan.get(), s);
       }
       SHT_CUDA(cudaEventRecord(r->planned, s));
       r->npairs = r->plan->npairs;

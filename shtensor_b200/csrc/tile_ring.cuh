@@ -54,7 +54,7 @@ constexpr int kRingCtas = 2;      // per SM
 
 // How the operands and C are addressed (from the expression, the same for every block):
 constexpr int kRingLinA = 1, kRingLinB = 2;  // element (row, k) at row * rs + k * ks, rs or ks 1; data 16-byte aligned
-constexpr int kRingKmA = 4, kRingKmB = 8;    // linear with ks == 1 (else rs == 1): stage layout with k fastest
+constexpr int kRingKmA = 4, kRingKmB = 8;    // stage layout with k fastest (linear: ks == 1, else rs == 1)
 constexpr int kRingLinR = 16, kRingLinC = 32;  // C rows / columns at index * stride
 
 struct RingArgs {
@@ -389,38 +389,78 @@ __device__ __forceinline__ void ring_copy_k(double* dst, const double* src, int 
   }
 }
 
-// offset of combined index idx of the modes xs[0 .. n) in a column-major block of extents d
-__device__ __forceinline__ int ring_gather(const int* d, const int* xs, int n, int idx) {
+// Any order of modes, or data that is not 16-byte aligned: a pair's elements copied one by one through
+// offsets (rows-fastest stage layout, no shift).  Lane d holds extent and stride of the block's mode d.
+//
+// Offset of combined index idx of the modes xs[0 .. n); all lanes take part.
+__device__ __forceinline__ int ring_digits(const int* xs, int n, int idx, int ext, int stride) {
   int off = 0;
   for (int t = 0; t < n; ++t) {
-    const int x = xs[t], e = d[x];
-    int st = 1;
-    for (int u = 0; u < x; ++u) st *= d[u];
-    const int q = idx / e;
-    off += (idx - q * e) * st;
+    const int x = xs[t];
+    const int e = __shfl_sync(0xffffffffu, ext, x), s = __shfl_sync(0xffffffffu, stride, x);
+    const int q = t + 1 < n ? idx / e : 0;  // the last digit is what is left
+    off += (idx - q * e) * s;
     idx = q;
   }
   return off;
 }
 
-// any order of modes, or data that is not 16-byte aligned: both offsets gathered (rows-fastest
-// stage layout, no shift)
-static __device__ __noinline__ void ring_copy_any(double* dst, const double* src, const int* d, const ModeMap* fm,
-                                                  const int* kx, int nk, int r0, int rows, int k0, int kc, int lane) {
-  int ro[2];
-#pragma unroll
-  for (int i = 0; i < 2; ++i) ro[i] = lane + 32 * i < rows ? ring_gather(d, fm->x, fm->n, r0 + lane + 32 * i) : -1;
-  // lane k tabulates the offset of k0 + k
-  const int mine = lane < kc ? ring_gather(d, kx, nk, k0 + lane) : 0;
-  for (int k = 0; k < kc; ++k) {
-    const double* s = src + __shfl_sync(0xffffffffu, mine, k);
-#pragma unroll
-    for (int i = 0; i < 2; ++i)
-      if (ro[i] >= 0) ring_cp8(dst + k * kRingPitchR + lane + 32 * i, s + ro[i]);
+// All chunks of one pair from stage st on; false when a wait ran out.  The extents are loaded and the row
+// offsets worked out once per pair (with that done per chunk, the extents loaded again for every mode, a
+// chunk took up to 9,000 cycles: abcd,cidj->abij, 281 GFLOP, 16.9 ms, now 13.1).  Lanes run along the rows
+// of one k, or (kfast: the contracted index's first mode is the block's fastest) along the k of one row,
+// two or four of them at a time when they are few.
+static __device__ __noinline__ bool ring_gather(RingSmem& sm, bool isb, bool kfast, const RingArgs* g, const double* src,
+                                                const int* dims, int r0, int rows, int K, int st, unsigned ph, int lane) {
+  const RingWait wait{&sm.abort, g->err, g->wait_limit};
+  const int order = isb ? g->mp.oB : g->mp.oA;
+  const ModeMap& fm = isb ? g->mp.col : g->mp.row;
+  const int* kx = isb ? g->mp.kk.y : g->mp.kk.x;
+  const int nk = g->mp.kk.n;
+  const int ext = lane < order ? dims[lane] : 1;
+  int stride = 1;
+  for (int d = 0; d + 1 < order; ++d) {
+    const int e = __shfl_sync(0xffffffffu, ext, d);
+    if (d < lane) stride *= e;
   }
+  // lane i: offsets of rows i and 32 + i
+  const int ra = ring_digits(fm.x, fm.n, r0 + lane, ext, stride);
+  const int rb = rows > 32 ? ring_digits(fm.x, fm.n, r0 + 32 + lane, ext, stride) : 0;
+  for (int k0 = 0; k0 < K; k0 += kRingK) {
+    const int kc = min(kRingK, K - k0);
+    const int ko = ring_digits(kx, nk, k0 + lane, ext, stride);  // lane k: offset of k0 + k
+    if (!wait(&sm.empty[st], ph ^ 1u)) return false;
+    // `inner` indices over 2^w lanes, 32 >> w outer ones at once
+    const int inner = kfast ? kc : min(rows, 32), outer = kfast ? rows : kc;
+    const int w = inner <= 8 ? 3 : inner <= 16 ? 4 : 5, step = 32 >> w;
+    const int i = lane & ((1 << w) - 1), o0 = lane >> w;
+    const int pitch = kfast ? kRingPitchK : kRingPitchR;
+    double* d = sm.stage[st][isb ? 1 : 0] + i + o0 * pitch;
+    const int mine = __shfl_sync(0xffffffffu, kfast ? ko : ra, i);
+    const double *s0 = src + mine, *s1 = src + rb;
+    const bool in0 = i < inner, in1 = !kfast && 32 + lane < rows;
+#pragma unroll 4
+    for (int o = 0; o < outer; o += step) {
+      const int at = o + o0;
+      int off = __shfl_sync(0xffffffffu, kfast ? ra : ko, at & 31);
+      if (kfast && o >= 32) off = __shfl_sync(0xffffffffu, rb, at & 31);
+      if (at < outer) {
+        if (in0) ring_cp8(d + o * pitch, s0 + off);
+        if (in1) ring_cp8(d + o * pitch + 32, s1 + off);
+      }
+    }
+    mbar_arrive_cp_async(&sm.full[st]);
+    if (++st == kRingStages) {
+      st = 0;
+      ph ^= 1u;
+    }
+  }
+  return true;
 }
 
-// One load warp per operand; both run this code.
+// One load warp per operand; both run this code.  Gather: some operand needs ring_gather (an instance of
+// its own: its code beside the linear copies' costs those 2 to 8%).
+template <bool Gather>
 __device__ __forceinline__ void ring_load(RingSmem& sm, bool isb, int lane, const RingWait& wait) {
   int st = 0;
   unsigned ph = 0, q = 0;
@@ -444,13 +484,21 @@ __device__ __forceinline__ void ring_load(RingSmem& sm, bool isb, int lane, cons
       const int rs = isb ? v.rsB : v.rsA, ks = isb ? v.ksB : v.ksA, par = isb ? v.parB : v.parA, K = v.K;
       __syncwarp();
       if (lane == 0) mbar_arrive(&sm.pempty[qs]);
+      if (Gather && !lin) {
+        ok = ring_gather(sm, isb, km, g, src, dims, r0, rows, K, st, ph, lane);
+        for (int k0 = 0; k0 < K; k0 += kRingK)
+          if (++st == kRingStages) {
+            st = 0;
+            ph ^= 1u;
+          }
+        continue;
+      }
       for (int k0 = 0; k0 < K; k0 += kRingK) {
         const int kc = min(kRingK, K - k0);
         if (!wait(&sm.empty[st], ph ^ 1u)) { ok = false; break; }
         double* d = sm.stage[st][isb ? 1 : 0];
         if (km) ring_copy_k(d, src + k0, rs, rows, kc, par, lane);
-        else if (lin) ring_copy_rows(d, src + (long long)k0 * ks, ks, rows, kc, par, lane);
-        else ring_copy_any(d, src, dims, isb ? &g->mp.col : &g->mp.row, isb ? g->mp.kk.y : g->mp.kk.x, g->mp.kk.n, r0, rows, k0, kc, lane);
+        else ring_copy_rows(d, src + (long long)k0 * ks, ks, rows, kc, par, lane);
         mbar_arrive_cp_async(&sm.full[st]);
         if (++st == kRingStages) {
           st = 0;
@@ -653,7 +701,7 @@ __device__ __forceinline__ void ring_multiply(RingSmem& sm, int warp, int lane, 
   }
 }
 
-template <int Kind>
+template <int Kind, bool Gather>
 __global__ void __launch_bounds__(kRingThreads, kRingCtas) k_tiles(const __grid_constant__ RingArgs g) {
   extern __shared__ __align__(16) unsigned char ring_smem[];
   RingSmem& sm = *reinterpret_cast<RingSmem*>(ring_smem);
@@ -679,7 +727,7 @@ __global__ void __launch_bounds__(kRingThreads, kRingCtas) k_tiles(const __grid_
   if (warp < kRingMmaWarps) {
     ring_multiply(sm, warp, lane, wait);
   } else {
-    if (warp < kRingMmaWarps + kRingLoadWarps) ring_load(sm, warp > kRingMmaWarps, lane, wait);
+    if (warp < kRingMmaWarps + kRingLoadWarps) ring_load<Gather>(sm, warp > kRingMmaWarps, lane, wait);
     else if (warp == kRingMmaWarps + kRingLoadWarps) ring_schedule<Kind>(g, sm, lane, wait);
   }
 }
