@@ -33,26 +33,37 @@ def timeout(call, *args, **kw):
     return str(ei.value)
 
 
+def long_waits(ctx):
+    # one C block of 16 pairs, each of which takes its tile a hundred chunks: the roles that run ahead wait for
+    # far longer than a poll
+    rng = np.random.default_rng(3)
+    A = W.build_tensor(rng, [[64], [3200] * 16], lambda c: np.ones(len(c[0]), bool), None, "normal")
+    B = W.build_tensor(rng, [[3200] * 16, [64]], lambda c: np.ones(len(c[0]), bool), None, "normal")
+    Ch = W.empty_tensor([[64], [64]])
+    want = oracle.contract(EXPR, 1.0, host(A), host(B), 0.0, host(Ch))
+    return dev(ctx, A), dev(ctx, B), dev(ctx, Ch), want.C.data
+
+
+EXPR = "ik, kj -> ij"
+
+
 @pytest.mark.parametrize("mode", FP64)
 def test_contract_times_out_and_recovers(one_poll, mode):
     ctx = one_poll
-    w = W.c1(seed=14, scale=0.25, occupancy=0.4)
-    A, B, C = dev(ctx, w.A), dev(ctx, w.B), dev(ctx, w.C)
-    sht.contract(ctx, w.expr, 1.0, A, B, 0.0, C, mode=mode)
+    A, B, C, want = long_waits(ctx)
+    sht.contract(ctx, EXPR, 1.0, A, B, 0.0, C, mode=mode)
     assert "split" not in timeout(ctx.stream_sync)
     ctx.stream_sync()  # reported once
     ctx.set_wait_limit(0)
-    sht.contract(ctx, w.expr, 1.0, A, B, 0.0, C, mode=mode)
-    want = oracle.contract(w.expr, 1.0, host(w.A), host(w.B), 0.0, host(w.C))
-    assert bits_equal(C.download(), want.C.data)
+    sht.contract(ctx, EXPR, 1.0, A, B, 0.0, C, mode=mode)
+    assert bits_equal(C.download(), want)
 
 
 def test_plan_and_graph_report_an_earlier_timeout(one_poll):
     import torch
     ctx = one_poll
-    w = W.c1(seed=14, scale=0.25, occupancy=0.4)
-    A, B, C = dev(ctx, w.A), dev(ctx, w.B), dev(ctx, w.C)
-    plan = sht.Plan(ctx, w.expr, A, B, C, mode=sht.Mode.BATCHED_FP64)
+    A, B, C, want = long_waits(ctx)
+    plan = sht.Plan(ctx, EXPR, A, B, C, mode=sht.Mode.BATCHED_FP64)
     s = torch.cuda.Stream()
     for graph in (False, True):
         plan.execute(1.0, 0.0, stream=s)
@@ -62,37 +73,35 @@ def test_plan_and_graph_report_an_earlier_timeout(one_poll):
     plan.execute(1.0, 0.0, stream=s, graph=True)
     s.synchronize()
     ctx.stream_sync()
-    want = oracle.contract(w.expr, 1.0, host(w.A), host(w.B), 0.0, host(w.C))
-    assert bits_equal(C.download(), want.C.data)
+    assert bits_equal(C.download(), want)
 
 
 def test_stack_of_large_blocks_times_out_and_recovers(one_poll):
+    # eight ops per resident CTA, each sixteen chunks long: tiles are claimed far ahead of their turn
     import torch
     ctx = one_poll
-    sa, sb, sc, n = [13, 32, 64], [9, 25, 64], [13, 9, 32, 25], 64
-    k = sht.Kernel(ctx, "iaP, jbP -> ijab", sa, sb, sc)
-    g = torch.Generator().manual_seed(3)
-    a, b = (torch.rand(n * int(np.prod(x)), dtype=torch.float64, generator=g).cuda() for x in (sa, sb))
-    c = torch.zeros(n * int(np.prod(sc)), dtype=torch.float64, device="cuda")
+    n, m, K = 8 * 296, 64, 512
+    k = sht.Kernel(ctx, EXPR, [m, K], [K, m], [m, m])
+    g = torch.Generator(device="cuda").manual_seed(3)
+    a, b = (torch.rand(n * m * K, dtype=torch.float64, device="cuda", generator=g) for _ in range(2))
+    c = torch.zeros(n * m * m, dtype=torch.float64, device="cuda")
     k.call(a, b, c, n)
     torch.cuda.synchronize()
     timeout(k.call, a, b, c, n)
     ctx.set_wait_limit(0)
     k.call(a, b, c, n)
     torch.cuda.synchronize()
-    want = torch.einsum("zPai, zPbj -> zbaji", a.view(n, *sa[::-1]), b.view(n, *sb[::-1])).reshape(-1)
-    # one rounding per product and sum of 64 terms on either side, all below 1
-    assert (c - want).abs().max().item() <= 2 * 64 * 64 * 2.0 ** -53
+    want = torch.bmm(b.view(n, m, K), a.view(n, K, m)).reshape(-1)
+    # 512 products and sums on either side, each rounded once, all terms below 1
+    assert (c - want).abs().max().item() <= 2 * K * K * 2.0 ** -53
 
 
 def test_served_request_times_out(one_poll):
     ctx = one_poll
-    w = W.c1(seed=14, scale=0.25, occupancy=0.4)
-    A, B, C = dev(ctx, w.A), dev(ctx, w.B), dev(ctx, w.C)
+    A, B, C, want = long_waits(ctx)
     with sht.Server(ctx) as srv:
-        msg = timeout(srv.wait, srv.submit(w.expr, 1.0, A, B, 0.0, C), 60)
+        msg = timeout(srv.wait, srv.submit(EXPR, 1.0, A, B, 0.0, C), 60)
         assert "tensor cores" not in msg
         ctx.set_wait_limit(0)
-        srv.wait(srv.submit(w.expr, 1.0, A, B, 0.0, C), 60)
-    want = oracle.contract(w.expr, 1.0, host(w.A), host(w.B), 0.0, host(w.C))
-    assert bits_equal(C.download(), want.C.data)
+        srv.wait(srv.submit(EXPR, 1.0, A, B, 0.0, C), 60)
+    assert bits_equal(C.download(), want)
