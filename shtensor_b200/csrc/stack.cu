@@ -4,7 +4,7 @@
 // and the asmjit AVX2 gather/FMA/scatter microkernel, :210-770).  The permutes are fused into the
 // operand reads and the per-element arithmetic is the XMM kernel's (k ascending, one fma each), so
 // results are bit-identical to the CPU restatement.  Three kernels:
-//   * blocks whose A and B fit in shared memory twice (kStagedBytes): a CTA takes one op after
+//   * blocks whose A and B fit in shared memory (staged_fits): a CTA takes one op after
 //     another, copies the next op's two blocks whole -- contiguous, whatever the index order --
 //     while it multiplies the current one from shared memory through offset tables built once;
 //     FP64 on the tensor cores (k_stack_dmma), FP32 with FFMA register tiles (k_stack_fma);
@@ -68,6 +68,7 @@ struct StagedArgs {
   int m, n, K;
   int mp, np, kp;          // padded table lengths
   int abytes, bbytes;      // one buffer of A, of B (128-byte multiples with room for the alignment)
+  int single;              // no room for two buffers: the next op's copies wait for the current op
   int lr;                  // FP32: lanes along rows (8, 16 or 32)
 };
 
@@ -161,13 +162,19 @@ __device__ __forceinline__ void staged_ops(const StagedArgs<T>& g, unsigned char
   };
   fetch(blockIdx.x, bufs);
   unsigned cur = 0;
-  for (long long op = blockIdx.x; op < g.nb_ops; op += gridDim.x, cur = both - cur) {
-    fetch(op + gridDim.x, bufs + both - cur);
-    asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+  for (long long op = blockIdx.x; op < g.nb_ops; op += gridDim.x) {
+    if (g.single) {
+      asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    } else {
+      fetch(op + gridDim.x, bufs + both - cur);
+      asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+    }
     __syncthreads();  // every thread's copies of this op (and, the first time, the tables)
     body(cur, cur + g.abytes, staged_shift(g.A + op * g.size_a), staged_shift(g.B + op * g.size_b),
          g.C + op * g.size_c);
-    __syncthreads();  // the buffer is refilled from the next turn on
+    __syncthreads();  // the buffer is refilled from here on
+    if (g.single) fetch(op + gridDim.x, bufs);
+    else cur = both - cur;
   }
   asm volatile("cp.async.wait_all;\n" ::: "memory");
 }
@@ -313,6 +320,34 @@ __global__ void __launch_bounds__(32 * kStagedWarpsMax) k_stack_fma(const __grid
   });
 }
 
+// Both blocks of an op at most this many bytes: two ops' buffers are then 48 KB, so that several CTAs share
+// an SM, which hides the copies' latency (four and more by shared memory; registers keep the eight-warp
+// instances at two or three).
+constexpr long long kStagedBytes = 24 * 1024, kStagedTables = 4096;
+// FP64 blocks whose free or contracted modes lie apart: as many as fit an SM, two ops' buffers up to
+// kStagedTwo.  The ring kernel can only gather such blocks element by element.  Measured, kil,ljk->ji,
+// 14x23x18 by 18x20x14 (86 KB), 2,258 ops: 183 us with a gathering tile, 223 us with the ring, 78 us staged;
+// abcd,dcij->abij 8x5x12x6 by 6x12x8x10, 2,761 ops: 310, 199, 133.
+constexpr long long kStagedTwo = 100 * 1024, kStagedApart = 200 * 1024;
+static long long staged_bytes(const sht_kernel* k, size_t es) { return (k->size_a + k->size_b) * (long long)es; }
+static bool modes_apart(const sht_kernel* k) {
+  auto apart = [](const std::vector<int>& v) { return !modes_consecutive(v.data(), (int)v.size()); };
+  return apart(k->maps.rowA) || apart(k->maps.colA) || apart(k->maps.colB) || apart(k->maps.rowB);
+}
+static bool staged_fits(const sht_kernel* k, size_t es) {
+  const long long most = es == 8 && modes_apart(k) ? kStagedApart : kStagedBytes;
+  return staged_bytes(k, es) <= most && k->m + k->n + k->k <= kStagedTables / 2;
+}
+// With fewer ops than SMs the ring kernel spreads an op's tiles over the chip, which from four tiles on is
+// the faster (iPa,jPb->ijab 21x14x27 by 8x14x24, one op, 27 tiles: 41.6 us staged, 10.5 with the ring;
+// acbd,cidj->abij 7x9x10x3 by 9x9x3x12, 2 ops, 4 tiles: 10.5 and 10.4; 10x12x6x10 by 12x9x10x2, one op, 2
+// tiles: 8.4 and 16.6).
+static bool use_staged(const sht_kernel* k, size_t es, long long nb_ops) {
+  if (!staged_fits(k, es)) return false;
+  if (staged_bytes(k, es) <= kStagedBytes || nb_ops >= k->ctx->num_sms) return true;
+  return ring_ntiles((int)k->m, kRingTile) * ring_ntiles((int)k->n, kRingTile) < 4;
+}
+
 static StagedModes staged_modes(const std::vector<int>& modes, const std::vector<int>& dims) {
   StagedModes m{};
   m.n = (int)modes.size();
@@ -352,6 +387,7 @@ static StagedArgs<T> staged_args(const sht_kernel* k, const StackArgs<T>& g, lon
   s.kp = (s.K + 3) & ~3;
   s.abytes = (int)((g.size_a * sizeof(T) + 16 + 127) & ~127ull);
   s.bbytes = (int)((g.size_b * sizeof(T) + 16 + 127) & ~127ull);
+  s.single = staged_bytes(k, sizeof(T)) > kStagedTwo;
   s.lr = 32;
   return s;
 }
@@ -401,8 +437,6 @@ static FmaShape pick_fma_shape(int m, int n, bool few) {
   return best;
 }
 
-static bool staged_fits(const sht_kernel* k, size_t es);
-
 // Host decisions of a kernel's calls that depend on its shape only.
 void stack_prepare(sht_kernel* k) {
   const bool f64 = k->dtype == SHT_F64;
@@ -419,18 +453,12 @@ void stack_prepare(sht_kernel* k) {
   k->swizzle = 4 * w[1] < 3 * w[0];  // it costs two integer instructions a read
 }
 
-// Both blocks of an op at most this many bytes: two ops' buffers are then 48 KB, and four CTAs or
-// more share an SM, which hides the copies' latency.
-constexpr long long kStagedBytes = 24 * 1024, kStagedTables = 4096;
-static bool staged_fits(const sht_kernel* k, size_t es) {
-  return (k->size_a + k->size_b) * (long long)es <= kStagedBytes && k->m + k->n + k->k <= kStagedTables / 2;
-}
-
 template <typename T, class Kernel>
 static void launch_staged(sht_kernel* k, const StagedArgs<T>& s, int groups, bool few, Kernel kernel, cudaStream_t st) {
   // a warp per group of the block; more where the copies would take a thread many turns
   const int warps = std::min(std::max(groups, few ? (s.abytes + s.bbytes) / 1024 : 0), kStagedWarpsMax);
-  const size_t smem = (((size_t)2 * (s.mp + s.np + s.kp) * 4 + 127) & ~(size_t)127) + 2 * (size_t)(s.abytes + s.bbytes);
+  const size_t smem = (((size_t)2 * (s.mp + s.np + s.kp) * 4 + 127) & ~(size_t)127) +
+                      (s.single ? 1 : 2) * (size_t)(s.abytes + s.bbytes);
   // resident CTAs by shared memory and by threads (a persistent wave; ops are strided over it)
   const long long per_sm = std::max<long long>(1, std::min<long long>({32, 227 * 1024 / (long long)(smem + 1024), 32 / warps}));
   const long long grid = std::min(s.nb_ops, per_sm * k->ctx->num_sms);
@@ -454,7 +482,7 @@ static void (*const kStackFma[4][4])(StagedArgs<float>) = {SHT_FMA(1, 2), SHT_FM
 static void stack_setup(int device) {
   static DeviceOnce once;
   once.run(device, [] {
-    const int big = 96 * 1024;  // buffers and tables of the largest staged shape
+    const int big = 222 * 1024;  // buffers and tables of the largest staged shape
     for (const auto& r : kStackDmma)
       for (auto* f : r) SHT_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
     for (const auto& r : kStackFma)
@@ -469,7 +497,7 @@ static bool few_ops(const sht_kernel* k, long long nb_ops) { return nb_ops <= k-
 static void launch_staged_op(sht_kernel* k, const StackArgs<double>& g, long long nb_ops, cudaStream_t st) {
   // the smallest tile that takes the block's rows and columns at once, up to 32 x 16; with few ops the
   // smallest whose groups a CTA's warps take at once
-  const bool few = few_ops(k, nb_ops);
+  const bool few = few_ops(k, nb_ops) || staged_bytes(k, 8) > kStagedBytes;
   int ri = k->m <= 8 ? 0 : k->m <= 16 ? 1 : 2, ci = k->n <= 8 ? 0 : 1;
   for (int t = 0, end = few ? 2 * ri + ci : 0; t < end; ++t)
     if (((k->m - 1) / (8 << t / 2) + 1) * ((k->n - 1) / (8 << t % 2) + 1) <= kStagedWarpsMax) {
@@ -586,7 +614,7 @@ static void launch_stack(sht_kernel* k, const T* a, const T* b, T* c, long long 
   g.A = a; g.B = b; g.C = c;
   g.size_a = k->size_a; g.size_b = k->size_b; g.size_c = k->size_c;
   stack_setup(k->ctx->device);
-  if (staged_fits(k, sizeof(T))) launch_staged_op(k, g, nb_ops, s);
+  if (use_staged(k, sizeof(T), nb_ops)) launch_staged_op(k, g, nb_ops, s);
   else launch_large(k, g, nb_ops, s);
 }
 
