@@ -68,7 +68,6 @@ struct StagedArgs {
   int m, n, K;
   int mp, np, kp;          // padded table lengths
   int abytes, bbytes;      // one buffer of A, of B (128-byte multiples with room for the alignment)
-  int single;              // no room for two buffers: the next op's copies wait for the current op
   int lr;                  // FP32: lanes along rows (8, 16 or 32)
 };
 
@@ -150,7 +149,9 @@ __device__ __forceinline__ T staged_read(const unsigned char* smem, unsigned buf
 
 // The op loop shared by both kernels: two buffers, the next op's copies in flight while body works.
 // body(where A's buffer starts in smem, where B's, byte shift of A's data in it, of B's, C).
-template <typename T, bool Swz, class Body>
+// Single: no room for two buffers, the next op's copies wait for the current op (an instance of its own: the
+// choice at run time cost 15% of small ops, 32x32 by 32x32, 200 ops).
+template <typename T, bool Swz, bool Single, class Body>
 __device__ __forceinline__ void staged_ops(const StagedArgs<T>& g, unsigned char* smem, Body body) {
   const unsigned bufs = smem_u32(smem), both = (unsigned)(g.abytes + g.bbytes);
   auto fetch = [&](long long op, unsigned at) {
@@ -162,19 +163,14 @@ __device__ __forceinline__ void staged_ops(const StagedArgs<T>& g, unsigned char
   };
   fetch(blockIdx.x, bufs);
   unsigned cur = 0;
-  for (long long op = blockIdx.x; op < g.nb_ops; op += gridDim.x) {
-    if (g.single) {
-      asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-    } else {
-      fetch(op + gridDim.x, bufs + both - cur);
-      asm volatile("cp.async.wait_group 1;\n" ::: "memory");
-    }
+  for (long long op = blockIdx.x; op < g.nb_ops; op += gridDim.x, cur = Single ? 0 : both - cur) {
+    if (!Single) fetch(op + gridDim.x, bufs + both - cur);
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(Single ? 0 : 1) : "memory");
     __syncthreads();  // every thread's copies of this op (and, the first time, the tables)
     body(cur, cur + g.abytes, staged_shift(g.A + op * g.size_a), staged_shift(g.B + op * g.size_b),
          g.C + op * g.size_c);
     __syncthreads();  // the buffer is refilled from here on
-    if (g.single) fetch(op + gridDim.x, bufs);
-    else cur = both - cur;
+    if (Single) fetch(op + gridDim.x, bufs);
   }
   asm volatile("cp.async.wait_all;\n" ::: "memory");
 }
@@ -187,7 +183,7 @@ __device__ __forceinline__ void staged_ops(const StagedArgs<T>& g, unsigned char
 // FP64: warps take groups of 8*ML x 8*NL of the C block (ML x NL fragments of m8n8k4; fragments past
 // the block multiply padding: the tensor pipe is not what bounds blocks of this size).
 constexpr int kStagedWarpsMax = 8;
-template <int ML, int NL, bool Scale, bool Swz>
+template <int ML, int NL, bool Scale, bool Swz, bool Single>
 __global__ void __launch_bounds__(32 * kStagedWarpsMax) k_stack_dmma(const __grid_constant__ StagedArgs<double> g) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   unsigned char* smem = smem_raw;
@@ -195,7 +191,7 @@ __global__ void __launch_bounds__(32 * kStagedWarpsMax) k_stack_dmma(const __gri
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   const int fr = lane >> 2, kq = lane & 3;
   const int gr = g.mp / (8 * ML), groups = gr * (g.np / (8 * NL));
-  staged_ops<double, Swz>(g, smem, [&](unsigned sa, unsigned sb, unsigned ea, unsigned eb, double* c) {
+  staged_ops<double, Swz, Single>(g, smem, [&](unsigned sa, unsigned sb, unsigned ea, unsigned eb, double* c) {
     for (int grp = warp; grp < groups; grp += nw) {
       const int r0 = grp % gr * (8 * ML) + fr, c0 = grp / gr * (8 * NL);
       unsigned pa[ML], pb[NL];
@@ -271,7 +267,7 @@ __global__ void __launch_bounds__(32 * kStagedWarpsMax) k_stack_fma(const __grid
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   const int lr = g.lr, lc = 32 / lr, r1 = lane & (lr - 1), c1 = lane / lr;
   const int gr = g.mp / (RM * lr), groups = gr * (g.np / (CN * lc));
-  staged_ops<float, Swz>(g, smem, [&](unsigned sa, unsigned sb, unsigned ea, unsigned eb, float* c) {
+  staged_ops<float, Swz, false>(g, smem, [&](unsigned sa, unsigned sb, unsigned ea, unsigned eb, float* c) {
     for (int grp = warp; grp < groups; grp += nw) {
       const int r0 = grp % gr * (RM * lr) + r1, c0 = grp / gr * (CN * lc) + c1;
       unsigned pa[RM], pb[CN];
@@ -327,15 +323,17 @@ constexpr long long kStagedBytes = 24 * 1024, kStagedTables = 4096;
 // FP64 blocks whose free or contracted modes lie apart: as many as fit an SM, two ops' buffers up to
 // kStagedTwo.  The ring kernel can only gather such blocks element by element.  Measured, kil,ljk->ji,
 // 14x23x18 by 18x20x14 (86 KB), 2,258 ops: 183 us with a gathering tile, 223 us with the ring, 78 us staged;
-// abcd,dcij->abij 8x5x12x6 by 6x12x8x10, 2,761 ops: 310, 199, 133.
+// abcd,dcij->abij 8x5x12x6 by 6x12x8x10, 2,761 ops: 310, 199, 133; one buffer, kil,ljk->ji 19x21x25 by
+// 25x23x19 (167 KB), 1,913 ops: 300, 425, 144.
 constexpr long long kStagedTwo = 100 * 1024, kStagedApart = 200 * 1024;
 static long long staged_bytes(const sht_kernel* k, size_t es) { return (k->size_a + k->size_b) * (long long)es; }
+static bool staged_single(const sht_kernel* k, size_t es) { return staged_bytes(k, es) > kStagedTwo; }
 static bool modes_apart(const sht_kernel* k) {
   auto apart = [](const std::vector<int>& v) { return !modes_consecutive(v.data(), (int)v.size()); };
   return apart(k->maps.rowA) || apart(k->maps.colA) || apart(k->maps.colB) || apart(k->maps.rowB);
 }
 static bool staged_fits(const sht_kernel* k, size_t es) {
-  const long long most = es == 8 && modes_apart(k) ? kStagedApart : kStagedBytes;
+  const long long most = es == 8 && k->apart ? kStagedApart : kStagedBytes;
   return staged_bytes(k, es) <= most && k->m + k->n + k->k <= kStagedTables / 2;
 }
 // With fewer ops than SMs the ring kernel spreads an op's tiles over the chip, which from four tiles on is
@@ -387,7 +385,6 @@ static StagedArgs<T> staged_args(const sht_kernel* k, const StackArgs<T>& g, lon
   s.kp = (s.K + 3) & ~3;
   s.abytes = (int)((g.size_a * sizeof(T) + 16 + 127) & ~127ull);
   s.bbytes = (int)((g.size_b * sizeof(T) + 16 + 127) & ~127ull);
-  s.single = staged_bytes(k, sizeof(T)) > kStagedTwo;
   s.lr = 32;
   return s;
 }
@@ -441,6 +438,7 @@ static FmaShape pick_fma_shape(int m, int n, bool few) {
 void stack_prepare(sht_kernel* k) {
   const bool f64 = k->dtype == SHT_F64;
   k->swizzle = false;
+  k->apart = modes_apart(k);
   if (!staged_fits(k, f64 ? 8 : 4)) return;
   const StagedModes ra = staged_modes(k->maps.rowA, k->sa), ka = staged_modes(k->maps.colA, k->sa);
   const StagedModes cb = staged_modes(k->maps.colB, k->sb), kb = staged_modes(k->maps.rowB, k->sb);
@@ -458,7 +456,7 @@ static void launch_staged(sht_kernel* k, const StagedArgs<T>& s, int groups, boo
   // a warp per group of the block; more where the copies would take a thread many turns
   const int warps = std::min(std::max(groups, few ? (s.abytes + s.bbytes) / 1024 : 0), kStagedWarpsMax);
   const size_t smem = (((size_t)2 * (s.mp + s.np + s.kp) * 4 + 127) & ~(size_t)127) +
-                      (s.single ? 1 : 2) * (size_t)(s.abytes + s.bbytes);
+                      (staged_single(k, sizeof(T)) ? 1 : 2) * (size_t)(s.abytes + s.bbytes);
   // resident CTAs by shared memory and by threads (a persistent wave; ops are strided over it)
   const long long per_sm = std::max<long long>(1, std::min<long long>({32, 227 * 1024 / (long long)(smem + 1024), 32 / warps}));
   const long long grid = std::min(s.nb_ops, per_sm * k->ctx->num_sms);
@@ -466,13 +464,16 @@ static void launch_staged(sht_kernel* k, const StagedArgs<T>& s, int groups, boo
   SHT_CUDA(cudaGetLastError());
 }
 
-// [tile][Scale * 2 + Swz]; FP64 tiles: 1, 2 or 4 fragment rows x 1 or 2 columns
-#define SHT_DMMA(ML, NL)                                                                                          \
-  {k_stack_dmma<ML, NL, false, false>, k_stack_dmma<ML, NL, false, true>, k_stack_dmma<ML, NL, true, false>,       \
-   k_stack_dmma<ML, NL, true, true>}
-static void (*const kStackDmma[6][4])(StagedArgs<double>) = {SHT_DMMA(1, 1), SHT_DMMA(1, 2), SHT_DMMA(2, 1),
+// [tile][Single * 4 + Scale * 2 + Swz]; FP64 tiles: 1, 2 or 4 fragment rows x 1 or 2 columns
+#define SHT_DMMA1(ML, NL, SINGLE)                                                                                  \
+  k_stack_dmma<ML, NL, false, false, SINGLE>, k_stack_dmma<ML, NL, false, true, SINGLE>,                           \
+      k_stack_dmma<ML, NL, true, false, SINGLE>, k_stack_dmma<ML, NL, true, true, SINGLE>
+#define SHT_DMMA(ML, NL) {SHT_DMMA1(ML, NL, false), SHT_DMMA1(ML, NL, true)}
+static void (*const kStackDmma[6][8])(StagedArgs<double>) = {SHT_DMMA(1, 1), SHT_DMMA(1, 2), SHT_DMMA(2, 1),
                                                              SHT_DMMA(2, 2), SHT_DMMA(4, 1), SHT_DMMA(4, 2)};
 #undef SHT_DMMA
+#undef SHT_DMMA1
+// [tile][Scale * 2 + Swz]
 #define SHT_FMA(RM, CN)                                                                                          \
   {k_stack_fma<RM, CN, false, false>, k_stack_fma<RM, CN, false, true>, k_stack_fma<RM, CN, true, false>,         \
    k_stack_fma<RM, CN, true, true>}
@@ -507,8 +508,8 @@ static void launch_staged_op(sht_kernel* k, const StackArgs<double>& g, long lon
     }
   const int rt = 8 << ri, ct = 8 << ci;
   const StagedArgs<double> s = staged_args(k, g, nb_ops, rt, ct);
-  launch_staged(k, s, (s.mp / rt) * (s.np / ct), few, kStackDmma[2 * ri + ci][(s.sc.alpha != 1.0 ? 2 : 0) + (k->swizzle ? 1 : 0)],
-                st);
+  const int instance = (staged_single(k, 8) ? 4 : 0) + (s.sc.alpha != 1.0 ? 2 : 0) + (k->swizzle ? 1 : 0);
+  launch_staged(k, s, (s.mp / rt) * (s.np / ct), few, kStackDmma[2 * ri + ci][instance], st);
 }
 static void launch_staged_op(sht_kernel* k, const StackArgs<float>& g, long long nb_ops, cudaStream_t st) {
   const bool few = few_ops(k, nb_ops);
