@@ -415,11 +415,15 @@ static void staged_wavefronts(const StagedModes& rows, const StagedModes& ks, in
     }
 }
 
-// FP32 register tile and lanes along rows: the least issue slots over the op's groups (products,
-// operand and table reads per k).  With few ops (an SM or more for each) the op's own time counts:
-// its groups run at once on up to kStagedWarpsMax warps, each k waiting about 40 cycles for its reads.
+// FP32 register tile and lanes along rows: the least issue slots over the op's groups (products, operand and
+// table reads per k).  With few ops (up to three for each SM) the op's own time counts too: its groups run at
+// once on up to kStagedWarpsMax warps, each k waiting about 40 cycles for its reads, and an SM has registers
+// for kStagedResident warps of the largest instances.  Measured, ik,kj->ij 30x60
+// by 60x30 (us, by issue slots alone / so): 149 ops 14.3 / 8.2, 300 ops 14.4 / 8.2.
 struct FmaShape { int rm, cn, lr; };
-static FmaShape pick_fma_shape(int m, int n, bool few) {
+constexpr double kFewPerSm = 3, kManyOps = 1e9;
+constexpr int kStagedResident = 16;
+static FmaShape pick_fma_shape(int m, int n, double ops_per_sm) {
   static const int tiles[][2] = {{1, 2}, {2, 4}, {4, 4}, {4, 8}};
   FmaShape best{4, 8, 32};
   double bc = 1e300;
@@ -428,7 +432,10 @@ static FmaShape pick_fma_shape(int m, int n, bool few) {
       const int rt = t[0] * lr, ct = t[1] * (32 / lr);
       const double groups = (double)((m + rt - 1) / rt) * (double)((n + ct - 1) / ct);
       const double k = t[0] * t[1] + 1.5 * (t[0] + t[1]) + 6;
-      const double c = few ? std::ceil(groups / kStagedWarpsMax) * (k + 40) : groups * k;
+      const double rounds = std::ceil(ops_per_sm / std::floor(kStagedResident / std::min(groups, (double)kStagedWarpsMax)));
+      const double latency = rounds * std::ceil(groups / kStagedWarpsMax) * (k + 40), issue = groups * k;
+      // an SM issues for four warps at once
+      const double c = ops_per_sm <= 1 ? latency : ops_per_sm <= kFewPerSm ? std::max(latency, ops_per_sm * issue / 4) : issue;
       if (c < bc) { bc = c; best = {t[0], t[1], lr}; }
     }
   return best;
@@ -444,7 +451,7 @@ void stack_prepare(sht_kernel* k) {
   const StagedModes cb = staged_modes(k->maps.colB, k->sb), kb = staged_modes(k->maps.rowB, k->sb);
   const int m = (int)k->m, n = (int)k->n, K = (int)k->k;
   // FP32 columns are the same for whole rows of lanes: only A's reads spread over the banks
-  const int lr = f64 ? 8 : pick_fma_shape(m, n, false).lr;
+  const int lr = f64 ? 8 : pick_fma_shape(m, n, kManyOps).lr;
   int w[2] = {0, 0};
   staged_wavefronts(ra, ka, m, K, f64, lr, w);
   if (f64) staged_wavefronts(cb, kb, n, K, f64, 8, w);
@@ -512,11 +519,14 @@ static void launch_staged_op(sht_kernel* k, const StackArgs<double>& g, long lon
   launch_staged(k, s, (s.mp / rt) * (s.np / ct), few, kStackDmma[2 * ri + ci][instance], st);
 }
 static void launch_staged_op(sht_kernel* k, const StackArgs<float>& g, long long nb_ops, cudaStream_t st) {
-  const bool few = few_ops(k, nb_ops);
-  const FmaShape f = pick_fma_shape((int)k->m, (int)k->n, few);
+  const double ops_per_sm = (double)nb_ops / k->ctx->num_sms;
+  const FmaShape f = pick_fma_shape((int)k->m, (int)k->n, ops_per_sm);
   const int rt = f.rm * f.lr, ct = f.cn * (32 / f.lr);
   StagedArgs<float> s = staged_args(k, g, nb_ops, rt, ct);
   s.lr = f.lr;
+  // more warps for the copies where every op stays resident
+  const int copy_warps = std::min(std::max((s.mp / rt) * (s.np / ct), (s.abytes + s.bbytes) / 1024), kStagedWarpsMax);
+  const bool few = ops_per_sm <= kFewPerSm && ops_per_sm <= kStagedResident / copy_warps;
   const int tile = f.rm == 1 ? 0 : f.rm == 2 ? 1 : f.cn == 4 ? 2 : 3;
   launch_staged(k, s, (s.mp / rt) * (s.np / ct), few, kStackFma[tile][(s.sc.alpha != 1.0f ? 2 : 0) + (k->swizzle ? 1 : 0)], st);
 }

@@ -43,3 +43,19 @@ def test_stack(ctx, expr, sa, sb, ops, shift):
             one = lambda h, n: h[op * n:(op + 1) * n].copy()  # noqa: E731
             want = oracle.kernel_xmm(expr, list(sa), list(sb), sc, alpha, beta, one(ha, na), one(hb, nb), one(hc, nc), 1)
             assert bits_equal(got[shift + op * nc:shift + (op + 1) * nc], want)
+
+
+@pytest.mark.parametrize("ops", [148, 149, 296, 300, 444, 445])
+def test_fp32_shapes_around_a_few_ops_per_sm(ctx, ops):
+    # the shape and the warps change with the ops for each SM (148 of them)
+    import torch
+    for sa, sb in (((30, 60), (60, 30)), ((63, 51), (51, 10)), ((64, 16), (16, 64))):
+        rng = np.random.default_rng(ops)
+        a, b = (rng.standard_normal(ops * s[0] * s[1]).astype(np.float32) for s in (sa, sb))
+        sc = [sa[0], sb[1]]
+        c = torch.empty(ops * sc[0] * sc[1], dtype=torch.float32, device="cuda")
+        sht.Kernel(ctx, "ik, kj -> ij", list(sa), list(sb), sc, dtype=np.float32).call(
+            torch.from_numpy(a).cuda(), torch.from_numpy(b).cuda(), c, ops)
+        want = oracle.kernel_xmm("ik, kj -> ij", list(sa), list(sb), sc, 1.0, 0.0, a, b,
+                                 np.zeros(c.numel(), np.float32), ops)
+        assert bits_equal(c.cpu().numpy(), want)
