@@ -1,4 +1,5 @@
-"""Benchmark of the block-sparse contraction (one JSON line on rank 0).
+"""Benchmark of the block-sparse contraction (one JSON line of a few KB on standard output, rank 0; the full
+record, with every configuration, serving phase and CPU leg, goes to standard error as one more line).
 
 Headline workload (``--workload c1``, the default): C[i,j,a,b] = sum_P A[i,a,P] B[j,b,P] at full
 size (i,j extent 64 in blocks of {5,9,13}; a,b 512 in {13,25,32}; P 2048 in {32,48,64}; 15%
@@ -407,6 +408,46 @@ def run_serving(args, sht, ctx, upload):
     return out
 
 
+# ------------------------------------------------------------------------------ the printed line
+def digits(x, n=6):
+    """x with its floats at n significant digits."""
+    if isinstance(x, float):
+        return float(f"{x:.{n}g}")
+    if isinstance(x, dict):
+        return {k: digits(v, n) for k, v in x.items()}
+    return [digits(v, n) for v in x] if isinstance(x, (list, tuple)) else x
+
+
+def summary_line(full):
+    """The full record with its long parts cut to their figures: a reader of the last few KB of the output
+    gets the whole line."""
+    def forms(fs):
+        return {k: {"ms_per_step": f["ms_per_step"], "gflops": f["gflops"], "exec_ms": f.get("exec_ms"),
+                    "frac": (f.get("roofline") or {}).get("frac"),
+                    **{e: (f.get("error_vs_oracle") or {}).get(e) for e in ("rel_fro", "bits_differ")}}
+                for k, f in fs.items()}
+
+    def served(s):
+        keep = ("p50_ms", "p99_ms", "gflops", "mean_batch", "mean_plan_ms", "completed", "failed")
+        return {ph: {k: s[ph][k] for k in keep if k in s[ph]} for ph in ("stream", "burst") if ph in s}
+
+    line = dict(full)
+    line["forms"] = forms(full["forms"])
+    line["configs"] = {k: forms(c["forms"]) for k, c in (full.get("configs") or {}).items()} or None
+    if full.get("serving"):
+        sv = full["serving"]
+        line["serving"] = {"alone_plain_gflops": sv["alone_plain"]["gflops"],
+                           **{k: served(sv[k]) for k in ("batched", "split") if k in sv}}
+    if full.get("cpu_baseline"):
+        line["cpu_baseline"] = {k: v for k, v in full["cpu_baseline"].items() if k != "legs"}
+    if full.get("kernels_per_step"):
+        line["kernels_per_step"] = {k: v["launches"] if isinstance(v, dict) else v
+                                    for k, v in dict(full["kernels_per_step"]).items()}
+    roof = {k: v for k, v in (full.get("roofline") or {}).items() if k != "traffic_source"}
+    line["roofline"] = roof or None
+    return digits(line)
+
+
 # ------------------------------------------------------------------------------ device legs
 FORMS = {"plain": 0, "batched": 1, "split": 2}
 
@@ -745,7 +786,8 @@ def run_ours(args):
             "gpu_launches_per_step": launches, "kernels_per_step": names or None,
             "configs": configs or None, "serving": serving,
         }
-        print(json.dumps(line), flush=True)
+        print(json.dumps(line), file=sys.stderr, flush=True)
+        print(json.dumps(summary_line(line)), flush=True)
     ctx.close()
     if world > 1:
         torch.distributed.destroy_process_group()
