@@ -1,11 +1,12 @@
 // batched.cu -- the FP64 forms of the block-sparse contraction: one persistent kernel (tile_ring.cuh)
 // over a work list.
 //
-// Every C block gets a tile shape from its matrix extents (m, n): by a padded-area model, or, in
+// Every C block gets a tile shape from its matrix extents (m, n): by a cost model (shape_cost), or, in
 // the batched form, by the autotuner's choice for its size class.  The plan builds a single work
-// list of (C block, tile, shape) items ordered by estimated cost, heaviest first; a persistent
-// grid (SMs x resident CTAs) claims items from an atomic counter.  Execute is a counter reset
-// plus one launch, and is what sht_plan_execute_graph captures.
+// list of items (ring_item: C block, first row and column, extents) ordered by estimated cost, heaviest
+// first; a persistent grid (SMs x resident CTAs) claims items from an atomic counter.  Execute is the
+// copy of operands whose modes lie apart (linear.cu), a counter reset and one launch, and is what
+// sht_plan_execute_graph captures.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -118,46 +119,16 @@ static HostPlanView host_view(sht_plan* p, cudaStream_t s) {
   return v;
 }
 
-// Work list: items (cblk, tile, shape), touched blocks sorted by cost (heaviest first), then
-// untouched blocks (beta scaling only).
-static void build_batched_work(sht_plan* p, const HostPlanView& v, const std::map<std::string, int>& shape_of,
-                               cudaStream_t s, const std::vector<char>* subset = nullptr,
-                               std::vector<int4>* out = nullptr) {
-  const long long nc = p->ncblk;
-  // order C blocks (not tiles) by cost, heaviest first; untouched blocks last
-  struct Blk { double cost; int c, sh, tiles; bool has; };
-  std::vector<Blk> blks;
-  blks.reserve(nc);
-  size_t ntouched = 0, nall = 0;
-  for (long long c = 0; c < nc; ++c) {
-    if (subset && !(*subset)[c]) continue;
-    auto it = shape_of.find(v.key[c].str());
-    const int sh = it != shape_of.end() ? it->second : model_shape((int)v.m[c], (int)v.n[c]);
-    const long long tm = ring_tm(sh), tn = ring_tn(sh);
-    const int tiles = (int)(((v.m[c] + tm - 1) / tm) * ((v.n[c] + tn - 1) / tn));
-    const bool has = v.pstart[c + 1] > v.pstart[c];
-    blks.push_back({has ? (double)tm * tn * (double)v.ksum[c] : -1.0, (int)c, sh, tiles, has});
-    nall += tiles;
-    if (has) ntouched += tiles;
-  }
-  std::stable_sort(blks.begin(), blks.end(), [](const Blk& a, const Blk& b) { return a.cost > b.cost; });
+// The tiles of the sampled C blocks in one shape, the blocks ordered by cost, heaviest first.
+static std::vector<int4> sampled_work(const HostPlanView& v, std::vector<long long> blocks, int sh) {
+  const int tm = ring_tm(sh), tn = ring_tn(sh);
+  std::stable_sort(blocks.begin(), blocks.end(), [&](long long a, long long b) { return v.ksum[a] > v.ksum[b]; });
   std::vector<int4> w;
-  w.reserve(nall);
-  for (const Blk& b : blks)
-    for (int t = 0; t < b.tiles; ++t)
-      w.push_back(ring_item(b.c, t, (int)v.m[b.c], (int)v.n[b.c], ring_tm(b.sh), ring_tn(b.sh)));
-  if (w.size() > (size_t)INT32_MAX) fail(SHT_ERR_UNSUPPORTED, "work list above 2^31 tiles");
-  if (out) {
-    *out = std::move(w);
-    return;
+  for (long long c : blocks) {
+    const int m = (int)v.m[c], n = (int)v.n[c], tiles = ring_ntiles(m, tm) * ring_ntiles(n, tn);
+    for (int t = 0; t < tiles; ++t) w.push_back(ring_item((int)c, t, m, n, tm, tn));
   }
-  p->bwork_touched = (long long)ntouched;
-  p->bwork = (long long)w.size();
-  p->d_bwork = PoolBuf(p->ctx->pool.get(), std::max<size_t>(w.size(), 1) * sizeof(int4), s);
-  if (!w.empty()) {
-    SHT_CUDA(cudaMemcpyAsync(p->d_bwork.ptr, w.data(), w.size() * sizeof(int4), cudaMemcpyHostToDevice, s));
-    SHT_CUDA(cudaStreamSynchronize(s));
-  }
+  return w;
 }
 
 static void launch_plan(sht_ctx* ctx, const RingArgs& g, cudaStream_t s) {
@@ -373,7 +344,8 @@ int batched_ctas_per_sm(sht_ctx* ctx) { return ring_grid(ctx) / ctx->num_sms; }
 // for plans.size() descriptors that the caller keeps unchanged until the launch completes (the
 // upload reads it asynchronously); `descs` and `counter` are allocated on `s` and must be held
 // as long.  ctas_per_sm (1..batched_ctas_per_sm) sets the persistent grid: fewer than the
-// maximum leaves room on every SM for the planning kernels of requests that arrive meanwhile.
+// maximum leaves room on every SM for small planning kernels of requests that arrive meanwhile (not
+// for k_match, whose CTAs take an SM's whole register file: it runs where a launch leaves SMs empty).
 // Returns the number of launch items.
 long long batched_multi_launch(sht_ctx* ctx, const std::vector<sht_plan*>& plans, const std::vector<SparseArgs>& args,
                                void* host_descs, PoolBuf& descs, PoolBuf& counter, int ctas_per_sm, cudaStream_t s) {
@@ -473,13 +445,13 @@ void autotune(sht_plan* p, const char* cache_file, cudaStream_t s) {
   bool changed = false;
   for (auto& kv : members) {
     if (ctx->tuned.count(kv.first)) continue;
-    std::vector<char> subset(p->ncblk, 0);
+    std::vector<long long> sampled;
     long long elems = 0;
     size_t taken = 0;
     const size_t stride = std::max<size_t>(1, kv.second.size() / 256);
     for (size_t i = 0; i < kv.second.size() && taken < 256; i += stride, ++taken) {
       const long long c = kv.second[i];
-      subset[c] = 1;
+      sampled.push_back(c);
       offs[c] = elems;
       elems += v.m[c] * v.n[c];
     }
@@ -488,9 +460,7 @@ void autotune(sht_plan* p, const char* cache_file, cudaStream_t s) {
     double best = 1e300;
     int best_sh = model_shape((int)v.m[kv.second[0]], (int)v.n[kv.second[0]]);
     for (int sh = 0; sh < kRingShapes; ++sh) {
-      std::map<std::string, int> forced{{kv.first, sh}};
-      std::vector<int4> items;
-      build_batched_work(p, v, forced, s, &subset, &items);
+      const std::vector<int4> items = sampled_work(v, sampled, sh);
       work = PoolBuf(pool, items.size() * sizeof(int4), s);
       SHT_CUDA(cudaMemcpyAsync(work.ptr, items.data(), items.size() * sizeof(int4), cudaMemcpyHostToDevice, s));
       SparseArgs sa = sparse_args(p, 1.0, 0.0);

@@ -305,8 +305,6 @@ struct MatchArgs {
   ModeMap row, col;
   const long long *idsA, *idsB, *idsC;
   long long nA, nB, nC;
-  const int* dimsA;
-  RecModes recA, recB;
   const double *normA, *normB;  // null: no screening
   double eps;
   int ncell, kspan;
