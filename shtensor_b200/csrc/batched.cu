@@ -19,6 +19,7 @@
 
 #include "contract.h"
 #include "device_common.cuh"
+#include "tile_pipe.cuh"
 #include "tile_ring.cuh"
 
 namespace sht {
@@ -62,6 +63,85 @@ static void launch_tiles(const RingArgs& g, int all, int grid, cudaStream_t s) {
   constexpr int linear = kRingLinA | kRingLinB;
   if ((all & linear) == linear) k_tiles<Kind, false><<<grid, kRingThreads, sizeof(RingSmem), s>>>(g);
   else k_tiles<Kind, true><<<grid, kRingThreads, sizeof(RingSmem), s>>>(g);
+  SHT_CUDA(cudaGetLastError());
+}
+
+// ------------------------------------------------------------------ small blocks
+// C blocks of at most 8 x 8: a warp each, one fragment, operands straight from memory, many warps in flight.
+// The persistent kernel pays about 1,100 cycles of hand-overs between its roles for every pair, however
+// small.  Same order per element: k ascending within a pair, pairs in order, one fma each.  Measured (us, a
+// tile kernel without roles / the persistent kernel / so): 100 x 100 cells of 3x3, 1M pairs 1324 / 2114 / 112;
+// 64 x 64 cells of 8x8, 262,144 pairs 534 / 610 / 51; 16 x 16 cells, 16,384 pairs of K 8 100 / 58 / 41, of K 64
+// 313 / 114 / 96.  With fewer C blocks a warp's chain of pairs is too long: they stay with the persistent kernel,
+// as do serving launches, whose requests share one kernel.
+template <bool Scale>
+__global__ void __launch_bounds__(256) k_small(const __grid_constant__ RingArgs g) {
+  const int lane = threadIdx.x & 31, fr = lane >> 2, kq = lane & 3;
+  const int nwarps = gridDim.x * 8;
+  for (int i = blockIdx.x * 8 + (threadIdx.x >> 5); i < g.nwork; i += nwarps) {
+    const int4 w = g.work[i];
+    const int c = w.x, mt = w.w & 0xffff, nt = w.w >> 16;
+    const int ps = g.pstart[c], pe = g.sc.alpha_zero ? ps : g.pstart[c + 1];
+    const int ext = lane < g.mp.oC ? g.dimsC[(long long)c * g.mp.oC + lane] : 1;
+    int stride = 1;
+    for (int d = 0; d + 1 < g.mp.oC; ++d) {
+      const int e = __shfl_sync(0xffffffffu, ext, d);
+      if (d < lane) stride *= e;
+    }
+    double* cr = g.C + g.offC[c] + ring_digits(g.mp.row.y, g.mp.row.n, fr, ext, stride);
+    const int co[2] = {ring_digits(g.mp.col.y, g.mp.col.n, 2 * kq, ext, stride),
+                       ring_digits(g.mp.col.y, g.mp.col.n, 2 * kq + 1, ext, stride)};
+    const bool in[2] = {fr < mt && 2 * kq < nt, fr < mt && 2 * kq + 1 < nt};
+    double acc[2] = {0.0, 0.0};
+    if (!g.sc.beta_zero) {
+#pragma unroll
+      for (int e = 0; e < 2; ++e)
+        if (in[e]) acc[e] = mul_rn(g.sc.beta, cr[co[e]]);
+    }
+    // rows and columns past the block read its first: they only reach elements that are not stored
+    const int ra = fr < mt ? fr : 0, rb = fr < nt ? fr : 0;
+    PairRec next{};
+    if (ps < pe) next = g.recs[ps];
+    for (int p = ps; p < pe; ++p) {
+      const PairRec r = next;
+      if (p + 1 < pe) next = g.recs[p + 1];
+      const double* a = g.A + r.offA + ra * r.rsA + kq * r.ksA;
+      const double* b = g.B + r.offB + rb * r.rsB + kq * r.ksB;
+#pragma unroll 4
+      for (int k = 0; k < r.K; k += 4) {
+        const bool live = k + kq < r.K;  // past the contracted extent: fma(-0, +0, c) == c
+        double af = live ? a[k * r.ksA] : -0.0;
+        const double bf = live ? b[k * r.ksB] : 0.0;
+        if (Scale && live) af = mul_rn(g.sc.alpha, af);
+        dmma884(acc, af, bf);
+      }
+    }
+#pragma unroll
+    for (int e = 0; e < 2; ++e)
+      if (in[e]) cr[co[e]] = acc[e];
+  }
+}
+
+constexpr int kSmallExtent = 8, kSmallK = 64;
+constexpr long long kSmallBlocks = 256;
+static bool small_blocks(const sht_plan* p) {
+  auto within = [](const sht_tensor* X, const std::vector<int>& modes, int most) {
+    long long e = 1;
+    for (int x : modes) {
+      e *= *std::max_element(X->bs[x].begin(), X->bs[x].end());
+      if (e > most) return false;
+    }
+    return true;
+  };
+  return p->ncblk >= kSmallBlocks && within(p->C, p->maps.rowC, kSmallExtent) && within(p->C, p->maps.colC, kSmallExtent) &&
+         within(p->A, p->maps.colA, kSmallK);
+}
+
+static void launch_small(sht_ctx* ctx, const RingArgs& g, cudaStream_t s) {
+  if (g.nwork <= 0) return;
+  const int grid = std::min((g.nwork + 7) / 8, ctx->num_sms * 8);
+  if (g.sc.alpha != 1.0) k_small<true><<<grid, 256, 0, s>>>(g);
+  else k_small<false><<<grid, 256, 0, s>>>(g);
   SHT_CUDA(cudaGetLastError());
 }
 
@@ -301,6 +381,7 @@ void ring_prepare(sht_plan* p, cudaStream_t s) {
     device_work_list(p, 0, 0, p->mode == SHT_MODE_BATCHED_FP64, s);
   }
   linear_prepare(p, s);
+  p->small_blocks = small_blocks(p);
   trace("work list", s);
 }
 
@@ -406,7 +487,10 @@ void ring_stack(sht_ctx* ctx, const SparseArgs& a, const PairRec& rec, const int
 
 void ring_launch(sht_plan* p, const SparseArgs& g, cudaStream_t s) {
   if (!g.sc.alpha_zero) linear_execute(p, s);
-  launch_plan(p->ctx, ring_args(p, g), s);
+  const RingArgs r = ring_args(p, g);
+  constexpr int linear = kRingLinA | kRingLinB;
+  if (p->small_blocks && (r.flags & linear) == linear) launch_small(p->ctx, r, s);
+  else launch_plan(p->ctx, r, s);
   trace("tile kernel", s);
 }
 

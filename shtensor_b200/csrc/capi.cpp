@@ -88,7 +88,8 @@ static void contract_split(sht_plan* p, double alpha, double beta, cudaStream_t 
   // The build reads the tensors' indices (complete: every index change in this library returns
   // after it is done) and, with screening, A's and B's values, which earlier work on s may still
   // write: only then does it wait for s.  So a contraction into a C whose pattern holds the
-  // product plans while the previous contraction on s still runs.
+  // product plans while the previous contraction on s still runs, as far as there is room: the counting
+  // kernel's cluster needs eight SMs with nothing resident, which a persistent kernel leaves in its tail.
   if (p->eps > 0.0) SHT_CUDA(cudaStreamWaitEvent(ps, lane.lane.start, 0));
   try {
     plan_build(p, ps, true);
@@ -125,7 +126,8 @@ static void prepare_mode(sht_plan* p, cudaStream_t s) {
 
 // The FP64 forms of sht_contract.  The build reads indices only (complete: every index change in
 // this library returns after it is done) unless it screens, so it runs on a lane stream and a
-// contraction into a C whose pattern holds the product plans while earlier work on s still runs.
+// contraction into a C whose pattern holds the product need not wait for earlier work on s (its counting
+// kernel waits for eight empty SMs, though, which a persistent kernel leaves in its tail).
 static void contract_fp64(sht_plan* p, double alpha, double beta, cudaStream_t s) {
   sht_ctx* ctx = p->ctx;
   LaneLease lane(ctx);

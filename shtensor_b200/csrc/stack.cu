@@ -464,7 +464,8 @@ static void launch_staged(sht_kernel* k, const StagedArgs<T>& s, int groups, boo
   const int warps = std::min(std::max(groups, few ? (s.abytes + s.bbytes) / 1024 : 0), kStagedWarpsMax);
   const size_t smem = (((size_t)2 * (s.mp + s.np + s.kp) * 4 + 127) & ~(size_t)127) +
                       (staged_single(k, sizeof(T)) ? 1 : 2) * (size_t)(s.abytes + s.bbytes);
-  // resident CTAs by shared memory and by threads (a persistent wave; ops are strided over it)
+  // CTAs by shared memory and by threads; ops are strided over them (registers may keep some of the grid for
+  // a second wave)
   const long long per_sm = std::max<long long>(1, std::min<long long>({32, 227 * 1024 / (long long)(smem + 1024), 32 / warps}));
   const long long grid = std::min(s.nb_ops, per_sm * k->ctx->num_sms);
   kernel<<<(unsigned)grid, 32 * warps, smem, st>>>(s);

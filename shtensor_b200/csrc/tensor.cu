@@ -330,7 +330,7 @@ __global__ void __launch_bounds__(kNormLanes) k_norm_chunks(const T* __restrict_
 
 // One warp per block: 32 chunk results are loaded together (the next 32 ahead of their use) and
 // folded one after another.  (One thread per block waited for a load per chunk: 110 us for blocks
-// of 1,300 chunks, 14 us so.)
+// of 1,300 chunks, 24 us so.)
 __global__ void k_norm_finish(const long long* __restrict__ cstart, const long long* __restrict__ nchunks, long long n,
                               const double* __restrict__ partial, int maxabs, double* __restrict__ out) {
   const int lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
