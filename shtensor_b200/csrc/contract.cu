@@ -288,15 +288,15 @@ constexpr int kMatchSums = 9;               // pairs, blocks, elements, tiles to
 
 // Whether counting is the faster path, from the mean pairs of a key.  Its cluster has eight SMs for the pairs
 // and the cells, and a warp lists the tiles of its cells one cell after another: about 0.27 ns a cell, 3.5 ns
-// a C block and 0.5 ns a pair beyond the launches.  The general path costs some 0.4 ms more to start with
+// a C block, 2.5 ns a block of the operands and 0.4 ns a pair beyond the launches.  The general path costs some 0.4 ms more to start with
 // and 0.1 ns a pair; with no C yet it writes the new pattern in steps of its own, 6 ns a block.  Measured, a
 // plan (us, general / counted): 8 keys, 512 x 512 cells, 2.1M pairs 905 / 2355; 512 keys, 512 x 512 cells,
 // 0.33M pairs 454 / 880; 100 keys, 100 x 100 cells, 1M pairs 493 / 458; 128 keys, 512 x 512 cells, 12,782
-// pairs 372 / 293.  A contraction into a new C, the same four: 7983 / 6739, 3015 / 2239, 2714 / 2610, 735 / 467.
-static bool match_pays(double cells, double pairs, bool new_c) {
+// pairs 372 / 293; one key, 200,000 cells, 99,731 pairs 525 / 833.  A contraction into a new C, the same four: 7983 / 6739, 3015 / 2239, 2714 / 2610, 735 / 467.
+static bool match_pays(double cells, double pairs, double operand_blocks, bool new_c) {
   const double blocks = std::min(cells, pairs);
-  const double counted = 0.27e-3 * cells + 3.5e-3 * blocks + 0.4e-3 * pairs;
-  return counted <= 470 + (new_c ? 150 + 6e-3 * blocks : 0);
+  const double counted = 0.27e-3 * cells + 3.5e-3 * blocks + 0.4e-3 * pairs + 2.5e-3 * operand_blocks;
+  return counted <= 500 + (new_c ? 150 + 6e-3 * blocks : 0);
 }
 
 struct MatchArgs {
@@ -883,7 +883,7 @@ void plan_match_begin(sht_plan* p, cudaStream_t s) {
   key_specs(p, ka, kb, kspan, cgrid);
   if (nA == 0 || nB == 0 || kspan > (unsigned long long)kMatchKeys || cgrid > (long double)kMatchCells) return;
   if (nA > (1 << 20) || nB > (1 << 20)) return;
-  if (!match_pays((double)cgrid, (double)nA * (double)nB / (double)kspan, nC == 0)) return;
+  if (!match_pays((double)cgrid, (double)nA * (double)nB / (double)kspan, (double)(nA + nB), nC == 0)) return;
   DevicePool* pool = p->ctx->pool.get();
   for (sht_tensor* t : {A, B, C}) tensor_touch(t, s);
   auto st = std::make_shared<MatchState>(p->ctx, s);
