@@ -67,14 +67,16 @@ static void launch_tiles(const RingArgs& g, int all, int grid, cudaStream_t s) {
 }
 
 // ------------------------------------------------------------------ small blocks
-// C blocks of at most 8 x 8: a warp each, one fragment, operands straight from memory, many warps in flight.
+// C blocks of at most 8 x 8 or 16 x 16: a warp each, one or four fragments, operands straight from memory, many
+// warps in flight.
 // The persistent kernel pays about 1,100 cycles of hand-overs between its roles for every pair, however
 // small.  Same order per element: k ascending within a pair, pairs in order, one fma each.  Measured (us, a
 // tile kernel without roles / the persistent kernel / so): 100 x 100 cells of 3x3, 1M pairs 1324 / 2114 / 112;
-// 64 x 64 cells of 8x8, 262,144 pairs 534 / 610 / 51; 16 x 16 cells, 16,384 pairs of K 8 100 / 58 / 41, of K 64
-// 313 / 114 / 96.  With fewer C blocks a warp's chain of pairs is too long: they stay with the persistent kernel,
-// as do serving launches, whose requests share one kernel.
-template <bool Scale>
+// 64 x 64 cells of 8x8, 262,144 pairs 534 / 610 / 49; of 16x16 and K 4 387 / 571 / 88; 16 x 16 cells of 8x8, 16,384
+// pairs of K 64 312 / 112 / 102.  With few C blocks a warp's chain of pairs is too long (16 x 16 cells of 16x16,
+// K 64: 314 / 122 / 196; 24 x 24 cells 185 / 95 / 82): those stay with the persistent kernel, as do serving launches,
+// whose requests share one kernel.
+template <int F, bool Scale>
 __global__ void __launch_bounds__(256) k_small(const __grid_constant__ RingArgs g) {
   const int lane = threadIdx.x & 31, fr = lane >> 2, kq = lane & 3;
   const int nwarps = gridDim.x * 8;
@@ -88,60 +90,100 @@ __global__ void __launch_bounds__(256) k_small(const __grid_constant__ RingArgs 
       const int e = __shfl_sync(0xffffffffu, ext, d);
       if (d < lane) stride *= e;
     }
-    double* cr = g.C + g.offC[c] + ring_digits(g.mp.row.y, g.mp.row.n, fr, ext, stride);
-    const int co[2] = {ring_digits(g.mp.col.y, g.mp.col.n, 2 * kq, ext, stride),
-                       ring_digits(g.mp.col.y, g.mp.col.n, 2 * kq + 1, ext, stride)};
-    const bool in[2] = {fr < mt && 2 * kq < nt, fr < mt && 2 * kq + 1 < nt};
-    double acc[2] = {0.0, 0.0};
+    double* cb = g.C + g.offC[c];
+    int ro[F], co[F][2];  // offsets in C, negative past the block
+    // rows and columns past the block read its first: they only reach elements that are not stored
+    int ra[F], rb[F];
+#pragma unroll
+    for (int f = 0; f < F; ++f) {
+      const int r = 8 * f + fr;
+      const int off = ring_digits(g.mp.row.y, g.mp.row.n, r, ext, stride);
+      ro[f] = r < mt ? off : -1;
+      ra[f] = r < mt ? r : 0;
+      rb[f] = r < nt ? r : 0;
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int s = 8 * f + 2 * kq + e, cs = ring_digits(g.mp.col.y, g.mp.col.n, s, ext, stride);
+        co[f][e] = s < nt ? cs : -1;
+      }
+    }
+    double acc[F][F][2] = {};
     if (!g.sc.beta_zero) {
 #pragma unroll
-      for (int e = 0; e < 2; ++e)
-        if (in[e]) acc[e] = mul_rn(g.sc.beta, cr[co[e]]);
+      for (int x = 0; x < F; ++x)
+#pragma unroll
+        for (int y = 0; y < F; ++y)
+#pragma unroll
+          for (int e = 0; e < 2; ++e)
+            if ((ro[x] | co[y][e]) >= 0) acc[x][y][e] = mul_rn(g.sc.beta, cb[ro[x] + co[y][e]]);
     }
-    // rows and columns past the block read its first: they only reach elements that are not stored
-    const int ra = fr < mt ? fr : 0, rb = fr < nt ? fr : 0;
     PairRec next{};
     if (ps < pe) next = g.recs[ps];
     for (int p = ps; p < pe; ++p) {
       const PairRec r = next;
       if (p + 1 < pe) next = g.recs[p + 1];
-      const double* a = g.A + r.offA + ra * r.rsA + kq * r.ksA;
-      const double* b = g.B + r.offB + rb * r.rsB + kq * r.ksB;
-#pragma unroll 4
-      for (int k = 0; k < r.K; k += 4) {
-        const bool live = k + kq < r.K;  // past the contracted extent: fma(-0, +0, c) == c
-        double af = live ? a[k * r.ksA] : -0.0;
-        const double bf = live ? b[k * r.ksB] : 0.0;
-        if (Scale && live) af = mul_rn(g.sc.alpha, af);
-        dmma884(acc, af, bf);
+      const double *a[F], *b[F];
+#pragma unroll
+      for (int f = 0; f < F; ++f) {
+        a[f] = g.A + r.offA + ra[f] * r.rsA + kq * r.ksA;
+        b[f] = g.B + r.offB + rb[f] * r.rsB + kq * r.ksB;
+      }
+      // four steps of four k: their loads are in flight together
+      for (int k0 = 0; k0 < r.K; k0 += 16) {
+        double af[4][F], bf[4][F];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int k = k0 + 4 * u;
+          const bool live = k + kq < r.K;  // past the contracted extent: fma(-0, +0, c) == c
+#pragma unroll
+          for (int f = 0; f < F; ++f) {
+            af[u][f] = live ? a[f][k * r.ksA] : -0.0;
+            bf[u][f] = live ? b[f][k * r.ksB] : 0.0;
+          }
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          if (k0 + 4 * u >= r.K) break;
+          if (Scale && k0 + 4 * u + kq < r.K) {
+#pragma unroll
+            for (int f = 0; f < F; ++f) af[u][f] = mul_rn(g.sc.alpha, af[u][f]);
+          }
+#pragma unroll
+          for (int x = 0; x < F; ++x)
+#pragma unroll
+            for (int y = 0; y < F; ++y) dmma884(acc[x][y], af[u][x], bf[u][y]);
+        }
       }
     }
 #pragma unroll
-    for (int e = 0; e < 2; ++e)
-      if (in[e]) cr[co[e]] = acc[e];
+    for (int x = 0; x < F; ++x)
+#pragma unroll
+      for (int y = 0; y < F; ++y)
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+          if ((ro[x] | co[y][e]) >= 0) cb[ro[x] + co[y][e]] = acc[x][y][e];
   }
 }
 
-constexpr int kSmallExtent = 8, kSmallK = 64;
-constexpr long long kSmallBlocks = 256;
-static bool small_blocks(const sht_plan* p) {
-  auto within = [](const sht_tensor* X, const std::vector<int>& modes, int most) {
+// Fragments along a side of the largest C block, 0: not for k_small.
+constexpr int kSmallExtent = 16, kSmallK = 64;
+static int small_blocks(const sht_plan* p) {
+  auto largest = [](const sht_tensor* X, const std::vector<int>& modes) {
     long long e = 1;
-    for (int x : modes) {
-      e *= *std::max_element(X->bs[x].begin(), X->bs[x].end());
-      if (e > most) return false;
-    }
-    return true;
+    for (int x : modes) e = std::min(e * X->bmax[x], 1LL << 31);
+    return e;
   };
-  return p->ncblk >= kSmallBlocks && within(p->C, p->maps.rowC, kSmallExtent) && within(p->C, p->maps.colC, kSmallExtent) &&
-         within(p->A, p->maps.colA, kSmallK);
+  const long long side = std::max(largest(p->C, p->maps.rowC), largest(p->C, p->maps.colC)), K = largest(p->A, p->maps.colA);
+  if (side > kSmallExtent || K > kSmallK || p->ncblk < (side > 8 ? 256 + 4 * K : 256)) return 0;
+  return side > 8 ? 2 : 1;
 }
 
-static void launch_small(sht_ctx* ctx, const RingArgs& g, cudaStream_t s) {
+static void launch_small(sht_ctx* ctx, const RingArgs& g, int f, cudaStream_t s) {
   if (g.nwork <= 0) return;
   const int grid = std::min((g.nwork + 7) / 8, ctx->num_sms * 8);
-  if (g.sc.alpha != 1.0) k_small<true><<<grid, 256, 0, s>>>(g);
-  else k_small<false><<<grid, 256, 0, s>>>(g);
+  const bool scale = g.sc.alpha != 1.0;
+  if (f == 1) (scale ? k_small<1, true> : k_small<1, false>)<<<grid, 256, 0, s>>>(g);
+  else (scale ? k_small<2, true> : k_small<2, false>)<<<grid, 256, 0, s>>>(g);
   SHT_CUDA(cudaGetLastError());
 }
 
@@ -489,7 +531,7 @@ void ring_launch(sht_plan* p, const SparseArgs& g, cudaStream_t s) {
   if (!g.sc.alpha_zero) linear_execute(p, s);
   const RingArgs r = ring_args(p, g);
   constexpr int linear = kRingLinA | kRingLinB;
-  if (p->small_blocks && (r.flags & linear) == linear) launch_small(p->ctx, r, s);
+  if (p->small_blocks && (r.flags & linear) == linear) launch_small(p->ctx, r, p->small_blocks, s);
   else launch_plan(p->ctx, r, s);
   trace("tile kernel", s);
 }

@@ -369,6 +369,7 @@ sht_status sht_tensor_create(sht_ctx* ctx, int order, const int* nblk, const int
       need(nblk[d] > 0, "every mode needs at least one block");
       t->nblk.push_back(nblk[d]);
       t->bs.emplace_back(block_sizes + pos, block_sizes + pos + nblk[d]);
+      t->bmax.push_back(*std::max_element(t->bs.back().begin(), t->bs.back().end()));
       for (int i = 0; i < nblk[d]; ++i) {
         need(block_sizes[pos + i] > 0, "block sizes must be positive");
         if (block_sizes[pos + i] > 32767) fail(SHT_ERR_UNSUPPORTED, "block extent above 32767 in one mode");

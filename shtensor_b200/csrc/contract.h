@@ -30,7 +30,7 @@ struct sht_plan {
   sht::PoolBuf d_cm, d_cn, d_cksum; // per C block: rows, columns, sum of the pairs' k
   sht::PoolBuf d_bwork;             // int4 per tile (ring_item; split plans: (C block, tile, ., .))
   sht::PoolBuf d_counter;           // work counter of the persistent FP64 kernel
-  bool small_blocks = false;        // k_small in place of the persistent kernel (batched.cu)
+  int small_blocks = 0;             // k_small in place of the persistent kernel (batched.cu)
   sht::PoolBuf lin_a, lin_b;        // operands in the order that kernel reads (linear.cu), when they need it
   long long bwork = 0, bwork_touched = 0;
   // split path: INT8 slices (K-major rows), row / column exponents, error words

@@ -141,7 +141,7 @@ static bool k_fast(const int* k, int nk) { return nk && k[0] == 0; }
 // Turns of the largest block of X along modes x of one index (the largest extents of all its modes).
 static double linear_turns(const sht_tensor* X, const int* x, int n, int each) {
   double largest = 1;
-  for (int t = 0; t < n; ++t) largest *= *std::max_element(X->bs[x[t]].begin(), X->bs[x[t]].end());
+  for (int t = 0; t < n; ++t) largest *= X->bmax[x[t]];
   return std::ceil(largest / each);
 }
 

@@ -208,6 +208,7 @@ struct sht_tensor {
   int order = 0;
   sht_dtype dtype = SHT_F64;
   std::vector<std::vector<int>> bs;
+  std::vector<int> bmax;  // largest block size of each mode
   std::vector<int> nblk;
   std::vector<int64_t> gstride;
   // host index (authoritative unless host_stale; read back under hmu: tensor_sync_host)

@@ -1,4 +1,4 @@
-"""Plans whose C blocks are all at most 8 x 8 (a warp for each) at the edges of that path, bit for bit against
+"""Plans whose C blocks are all at most 8 x 8 or 16 x 16 (a warp for each) at the edges of that path, bit for bit against
 the oracle (the kernel does the oracle's fma chain, so the bound is zero)."""
 import numpy as np
 import pytest
@@ -12,15 +12,20 @@ from tests.test_gpu_tiles import dev, host
 pytestmark = pytest.mark.gpu
 
 # expression, extents and number of blocks per mode: one element; every row, column and contracted extent
-# around a step of four; both modes fastest; several modes an index; modes apart; 255 and 256 C blocks; C
-# blocks of 9 rows, and a contracted extent of 65, take the general kernel
+# around a step of four and of sixteen; both modes fastest; several modes an index; modes apart; 255 and 256
+# C blocks, and the 316 that blocks of 9 and more need at K 15; a contracted extent of 65, and 17 rows, take the
+# general kernel
 CASES = [
     ("ik, kj -> ij", {"i": ([1], 16), "k": ([1], 5), "j": ([1], 16)}),
     ("ik, kj -> ij", {"i": ([1, 7, 8], 17), "k": ([1, 3, 4, 5, 8], 9), "j": ([1, 2, 7, 8], 16)}),
     ("ki, jk -> ji", {"i": ([1, 7, 8], 17), "k": ([1, 3, 4, 5, 33], 9), "j": ([1, 2, 7, 8], 16)}),
     ("ik, kj -> ij", {"i": ([8], 16), "k": ([63, 64], 4), "j": ([5], 16)}),
     ("ik, kj -> ij", {"i": ([8], 16), "k": ([64, 65], 4), "j": ([5], 16)}),
-    ("ik, kj -> ij", {"i": ([9, 8], 16), "k": ([5], 4), "j": ([5], 16)}),
+    ("ik, kj -> ij", {"i": ([9, 8], 18), "k": ([5], 4), "j": ([5], 18)}),
+    ("ik, kj -> ij", {"i": ([1, 9, 15, 16], 20), "k": ([1, 13, 15], 5), "j": ([7, 8, 9, 16], 19)}),
+    ("ki, jk -> ji", {"i": ([16], 25), "k": ([15, 16, 17, 33, 64], 5), "j": ([2, 16], 25)}),
+    ("ik, kj -> ij", {"i": ([9], 15), "k": ([15], 3), "j": ([16], 21)}),
+    ("ik, kj -> ij", {"i": ([9, 17], 25), "k": ([15], 3), "j": ([16], 25)}),
     ("ik, kj -> ij", {"i": ([3], 15), "k": ([5], 4), "j": ([6], 17)}),
     ("ijl, lkm -> kimj", {"i": ([1, 2], 5), "j": ([2, 4], 4), "l": ([3, 6], 4), "k": ([2, 3], 4), "m": ([1, 2], 4)}),
     ("ilj, kl -> jik", {"i": ([1, 2], 6), "j": ([2, 4], 6), "l": ([3, 6], 4), "k": ([5, 8], 8)}),
