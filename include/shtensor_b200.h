@@ -228,7 +228,7 @@ typedef struct {
   size_t reserve_bytes;  /* pool bytes that admission leaves free (0 = none) */
   int planners;          /* planner threads, each with its own stream (0 = 8) */
   int ctas_per_sm;       /* persistent CTAs per SM of a batched serving launch (0 = the most
-                            that fit minus one, leaving room for planning kernels) */
+                            that fit minus one, leaving room for small planning kernels) */
   int mode;              /* 0 or SHT_MODE_BATCHED_FP64: batched FP64; SHT_MODE_SPLIT: split
                             precision.  One launch holds requests of one form (and, in split
                             form, one slice count and reassembly instance). */
