@@ -79,8 +79,8 @@ static void launch_tiles(const RingArgs& g, int all, int grid, cudaStream_t s) {
 template <int F, bool Scale>
 __global__ void __launch_bounds__(256) k_small(const __grid_constant__ RingArgs g) {
   const int lane = threadIdx.x & 31, fr = lane >> 2, kq = lane & 3;
-  const int nwarps = gridDim.x * 8;
-  for (int i = blockIdx.x * 8 + (threadIdx.x >> 5); i < g.nwork; i += nwarps) {
+  // unsigned: nwork is below 2^31, so that the last step does not wrap
+  for (unsigned i = blockIdx.x * 8 + (threadIdx.x >> 5); i < (unsigned)g.nwork; i += gridDim.x * 8) {
     const int4 w = g.work[i];
     const int c = w.x, mt = w.w & 0xffff, nt = w.w >> 16;
     const int ps = g.pstart[c], pe = g.sc.alpha_zero ? ps : g.pstart[c + 1];
@@ -180,7 +180,7 @@ static int small_blocks(const sht_plan* p) {
 
 static void launch_small(sht_ctx* ctx, const RingArgs& g, int f, cudaStream_t s) {
   if (g.nwork <= 0) return;
-  const int grid = std::min((g.nwork + 7) / 8, ctx->num_sms * 8);
+  const int grid = (int)std::min((g.nwork + 7LL) / 8, ctx->num_sms * 8LL);
   const bool scale = g.sc.alpha != 1.0;
   if (f == 1) (scale ? k_small<1, true> : k_small<1, false>)<<<grid, 256, 0, s>>>(g);
   else (scale ? k_small<2, true> : k_small<2, false>)<<<grid, 256, 0, s>>>(g);

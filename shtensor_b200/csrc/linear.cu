@@ -186,6 +186,7 @@ void linear_execute(sht_plan* p, cudaStream_t s) {
   long long turns[2] = {0, 0};
   auto add = [&](const PoolBuf& buf, const sht_tensor* X, const ModeMap& fm, const int* k) {
     if (!buf.ptr) return;
+    if ((size_t)X->nnz * 8 > buf.bytes) fail(SHT_ERR_STATE, "an operand's pattern grew after the plan was made");
     const int nk = p->tmaps.kk.n;
     const bool kf = k_fast(k, nk);
     LinearArgs& a = g.x[n];

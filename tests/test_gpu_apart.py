@@ -109,3 +109,15 @@ def test_served_together_with_linear_requests(ctx):
     for e, A, B, C0, _, _, c, alpha in jobs:
         want = oracle.contract(e, alpha, host(A), host(B), 0.5, host(C0))
         assert bits_equal(c.download(), want.C.data)
+
+
+def test_operand_reserved_larger_after_the_plan(ctx):
+    # the plan's copy of the operand has the size of its pattern at creation
+    A, B, C0 = case("kil, ljk -> ji", 0.6)
+    a, b, c = dev(ctx, A), dev(ctx, B), dev(ctx, C0)
+    plan = sht.Plan(ctx, "kil, ljk -> ji", a, b, c)
+    a.reserve_all()
+    with pytest.raises(sht.ShtError) as ei:
+        plan.execute(1.0, 0.0)
+    assert ei.value.status == sht.Status.ERR_STATE
+    plan.close()
