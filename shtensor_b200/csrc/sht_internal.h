@@ -198,6 +198,8 @@ struct sht_kernel {
   sht_dtype dtype = SHT_F64;
   sht_kernel_type type = SHT_KERNEL_XMM;
   int64_t m = 0, n = 0, k = 0, size_a = 0, size_b = 0, size_c = 0;
+  ShtMaps staged;        // maps with the rows and the columns in C's order (stack_prepare)
+  bool scattered = false;  // C's fastest mode leads neither its rows nor its columns in `maps` (stack_prepare)
   bool apart = false;    // free or contracted modes of a block that do not follow one another (stack_prepare)
   bool swizzle = false;  // layout of the blocks staged in shared memory (stack_prepare)
 };
