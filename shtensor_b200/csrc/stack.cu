@@ -150,8 +150,7 @@ __device__ __forceinline__ T staged_read(const unsigned char* smem, unsigned buf
 
 // The op loop shared by both kernels: two buffers, the next op's copies in flight while body works.
 // body(where A's buffer starts in smem, where B's, byte shift of A's data in it, of B's, C).
-// Single: no room for two buffers, the next op's copies wait for the current op (an instance of its own: the
-// choice at run time cost 15% of small ops, 32x32 by 32x32, 200 ops).
+// Single: no room for two buffers, the next op's copies wait for the current op.
 template <typename T, bool Swz, bool Single, class Body>
 __device__ __forceinline__ void staged_ops(const StagedArgs<T>& g, unsigned char* smem, Body body) {
   const unsigned bufs = smem_u32(smem), both = (unsigned)(g.abytes + g.bbytes);
@@ -184,7 +183,11 @@ __device__ __forceinline__ void staged_ops(const StagedArgs<T>& g, unsigned char
 // FP64: warps take groups of 8*ML x 8*NL of the C block (ML x NL fragments of m8n8k4; fragments past
 // the block multiply padding: the tensor pipe is not what bounds blocks of this size).
 constexpr int kStagedWarpsMax = 8;
-template <int ML, int NL, bool Scale, bool Swz, bool Single>
+// Instances: one CTA an op, the next op's copies in flight (kStagedWhole); several CTAs share an op's groups
+// (kStagedSliced); the same with one buffer (kStagedSingle).  What the last two need at run time costs the first
+// up to 18% of small ops.
+constexpr int kStagedWhole = 0, kStagedSliced = 1, kStagedSingle = 2;
+template <int ML, int NL, bool Scale, bool Swz, int Kind>
 __global__ void __launch_bounds__(32 * kStagedWarpsMax) k_stack_dmma(const __grid_constant__ StagedArgs<double> g) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   unsigned char* smem = smem_raw;
@@ -192,8 +195,9 @@ __global__ void __launch_bounds__(32 * kStagedWarpsMax) k_stack_dmma(const __gri
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   const int fr = lane >> 2, kq = lane & 3;
   const int gr = g.mp / (8 * ML), groups = gr * (g.np / (8 * NL));
-  staged_ops<double, Swz, Single>(g, smem, [&](unsigned sa, unsigned sb, unsigned ea, unsigned eb, double* c) {
-    for (int grp = warp; grp < groups; grp += nw) {
+  const int g0 = Kind ? warp + nw * blockIdx.y : warp, gstep = Kind ? nw * gridDim.y : nw;
+  staged_ops<double, Swz, Kind == kStagedSingle>(g, smem, [&](unsigned sa, unsigned sb, unsigned ea, unsigned eb, double* c) {
+    for (int grp = g0; grp < groups; grp += gstep) {
       const int r0 = grp % gr * (8 * ML) + fr, c0 = grp / gr * (8 * NL);
       unsigned pa[ML], pb[NL];
 #pragma unroll
@@ -260,7 +264,7 @@ __global__ void __launch_bounds__(32 * kStagedWarpsMax) k_stack_dmma(const __gri
 
 // FP32: warps take groups of RM*lr rows x CN*(32/lr) columns; a lane has RM rows lr apart and CN
 // columns 32/lr apart, so that its stores run along the rows.
-template <int RM, int CN, bool Scale, bool Swz>
+template <int RM, int CN, bool Scale, bool Swz, int Kind>
 __global__ void __launch_bounds__(32 * kStagedWarpsMax) k_stack_fma(const __grid_constant__ StagedArgs<float> g) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   unsigned char* smem = smem_raw;
@@ -268,8 +272,9 @@ __global__ void __launch_bounds__(32 * kStagedWarpsMax) k_stack_fma(const __grid
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   const int lr = g.lr, lc = 32 / lr, r1 = lane & (lr - 1), c1 = lane / lr;
   const int gr = g.mp / (RM * lr), groups = gr * (g.np / (CN * lc));
+  const int g0 = Kind ? warp + nw * blockIdx.y : warp, gstep = Kind ? nw * gridDim.y : nw;
   staged_ops<float, Swz, false>(g, smem, [&](unsigned sa, unsigned sb, unsigned ea, unsigned eb, float* c) {
-    for (int grp = warp; grp < groups; grp += nw) {
+    for (int grp = g0; grp < groups; grp += gstep) {
       const int r0 = grp % gr * (RM * lr) + r1, c0 = grp / gr * (CN * lc) + c1;
       unsigned pa[RM], pb[CN];
 #pragma unroll
@@ -475,34 +480,41 @@ void stack_prepare(sht_kernel* k) {
   k->swizzle = 4 * w[1] < 3 * w[0];  // it costs two integer instructions a read
 }
 
+// kernels: [kind][Scale * 2 + Swz] of the tile; groups: of an op
 template <typename T, class Kernel>
-static void launch_staged(sht_kernel* k, const StagedArgs<T>& s, int groups, bool few, Kernel kernel, cudaStream_t st) {
+static void launch_staged(sht_kernel* k, const StagedArgs<T>& s, int groups, bool few, const Kernel* kernels,
+                          cudaStream_t st) {
   // a warp per group of the block; more where the copies would take a thread many turns
   const int warps = std::min(std::max(groups, few ? (s.abytes + s.bbytes) / 1024 : 0), kStagedWarpsMax);
+  const bool single = staged_single(k, sizeof(T));
   const size_t smem = (((size_t)2 * (s.mp + s.np + s.kp) * 4 + 127) & ~(size_t)127) +
-                      (staged_single(k, sizeof(T)) ? 1 : 2) * (size_t)(s.abytes + s.bbytes);
+                      (single ? 1 : 2) * (size_t)(s.abytes + s.bbytes);
   // CTAs by shared memory and by threads; ops are strided over them (registers may keep some of the grid for
   // a second wave)
   const long long per_sm = std::max<long long>(1, std::min<long long>({32, 227 * 1024 / (long long)(smem + 1024), 32 / warps}));
   const long long grid = std::min(s.nb_ops, per_sm * k->ctx->num_sms);
-  kernel<<<(unsigned)grid, 32 * warps, smem, st>>>(s);
+  // Few ops of many groups: several CTAs share an op, each with its two blocks staged.  Measured (us, a tile for
+  // each CTA / one CTA an op / so): FP64 ik,kj->ij 143x5 by 5x288, 22 ops 9.4 / 17.2 / 8.5; FP32
+  // Pia,Pjb->abij 4x29x26 by 4x28x20, 5 ops 18.8 / 96.6 / 10.5.
+  const long long slices = std::min<long long>((groups + warps - 1) / warps, per_sm * k->ctx->num_sms / s.nb_ops);
+  const int kind = single ? kStagedSingle : slices > 1 ? kStagedSliced : kStagedWhole;
+  kernels[4 * kind + (s.sc.alpha != 1.0 ? 2 : 0) + (k->swizzle ? 1 : 0)]<<<
+      dim3((unsigned)grid, (unsigned)std::max<long long>(slices, 1)), 32 * warps, smem, st>>>(s);
   SHT_CUDA(cudaGetLastError());
 }
 
-// [tile][Single * 4 + Scale * 2 + Swz]; FP64 tiles: 1, 2 or 4 fragment rows x 1 or 2 columns
-#define SHT_DMMA1(ML, NL, SINGLE)                                                                                  \
-  k_stack_dmma<ML, NL, false, false, SINGLE>, k_stack_dmma<ML, NL, false, true, SINGLE>,                           \
-      k_stack_dmma<ML, NL, true, false, SINGLE>, k_stack_dmma<ML, NL, true, true, SINGLE>
-#define SHT_DMMA(ML, NL) {SHT_DMMA1(ML, NL, false), SHT_DMMA1(ML, NL, true)}
-static void (*const kStackDmma[6][8])(StagedArgs<double>) = {SHT_DMMA(1, 1), SHT_DMMA(1, 2), SHT_DMMA(2, 1),
-                                                             SHT_DMMA(2, 2), SHT_DMMA(4, 1), SHT_DMMA(4, 2)};
+// [tile][kind * 4 + Scale * 2 + Swz]; FP64 tiles: 1, 2 or 4 fragment rows x 1 or 2 columns
+#define SHT_KIND(K, X, Y, KIND) \
+  K<X, Y, false, false, KIND>, K<X, Y, false, true, KIND>, K<X, Y, true, false, KIND>, K<X, Y, true, true, KIND>
+#define SHT_DMMA(ML, NL)                                                                                           \
+  {SHT_KIND(k_stack_dmma, ML, NL, kStagedWhole), SHT_KIND(k_stack_dmma, ML, NL, kStagedSliced),                     \
+   SHT_KIND(k_stack_dmma, ML, NL, kStagedSingle)}
+static void (*const kStackDmma[6][12])(StagedArgs<double>) = {SHT_DMMA(1, 1), SHT_DMMA(1, 2), SHT_DMMA(2, 1),
+                                                              SHT_DMMA(2, 2), SHT_DMMA(4, 1), SHT_DMMA(4, 2)};
+#define SHT_FMA(RM, CN) {SHT_KIND(k_stack_fma, RM, CN, kStagedWhole), SHT_KIND(k_stack_fma, RM, CN, kStagedSliced)}
+static void (*const kStackFma[4][8])(StagedArgs<float>) = {SHT_FMA(1, 2), SHT_FMA(2, 4), SHT_FMA(4, 4), SHT_FMA(4, 8)};
+#undef SHT_KIND
 #undef SHT_DMMA
-#undef SHT_DMMA1
-// [tile][Scale * 2 + Swz]
-#define SHT_FMA(RM, CN)                                                                                          \
-  {k_stack_fma<RM, CN, false, false>, k_stack_fma<RM, CN, false, true>, k_stack_fma<RM, CN, true, false>,         \
-   k_stack_fma<RM, CN, true, true>}
-static void (*const kStackFma[4][4])(StagedArgs<float>) = {SHT_FMA(1, 2), SHT_FMA(2, 4), SHT_FMA(4, 4), SHT_FMA(4, 8)};
 #undef SHT_FMA
 
 static void stack_setup(int device) {
@@ -533,8 +545,7 @@ static void launch_staged_op(sht_kernel* k, const StackArgs<double>& g, long lon
     }
   const int rt = 8 << ri, ct = 8 << ci;
   const StagedArgs<double> s = staged_args(k, g, nb_ops, rt, ct);
-  const int instance = (staged_single(k, 8) ? 4 : 0) + (s.sc.alpha != 1.0 ? 2 : 0) + (k->swizzle ? 1 : 0);
-  launch_staged(k, s, (s.mp / rt) * (s.np / ct), few, kStackDmma[2 * ri + ci][instance], st);
+  launch_staged(k, s, (s.mp / rt) * (s.np / ct), few, kStackDmma[2 * ri + ci], st);
 }
 static void launch_staged_op(sht_kernel* k, const StackArgs<float>& g, long long nb_ops, cudaStream_t st) {
   const double ops_per_sm = (double)nb_ops / k->ctx->num_sms;
@@ -546,7 +557,7 @@ static void launch_staged_op(sht_kernel* k, const StackArgs<float>& g, long long
   const int copy_warps = std::min(std::max((s.mp / rt) * (s.np / ct), (s.abytes + s.bbytes) / 1024), kStagedWarpsMax);
   const bool few = ops_per_sm <= kFewPerSm && ops_per_sm <= kStagedResident / copy_warps;
   const int tile = f.rm == 1 ? 0 : f.rm == 2 ? 1 : f.cn == 4 ? 2 : 3;
-  launch_staged(k, s, (s.mp / rt) * (s.np / ct), few, kStackFma[tile][(s.sc.alpha != 1.0f ? 2 : 0) + (k->swizzle ? 1 : 0)], st);
+  launch_staged(k, s, (s.mp / rt) * (s.np / ct), few, kStackFma[tile], st);
 }
 
 // ------------------------------------------------------------------ larger blocks
