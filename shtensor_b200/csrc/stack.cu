@@ -6,7 +6,8 @@
 // results are bit-identical to the CPU restatement.  Three kernels:
 //   * blocks whose A and B fit in shared memory (staged_fits): a CTA takes one op after
 //     another, copies the next op's two blocks whole -- contiguous, whatever the index order --
-//     while it multiplies the current one from shared memory through offset tables built once;
+//     while it multiplies the current one from shared memory through offset tables built once
+//     (with few ops several CTAs share one);
 //     FP64 on the tensor cores (k_stack_dmma), FP32 with FFMA register tiles (k_stack_fma);
 //   * larger FP64 blocks: the ring tile kernel (tile_ring.cuh), one pair per C block;
 //   * larger FP32 blocks: the gathering tile (tile_core.cuh).
